@@ -272,15 +272,17 @@ k_wgrad_mid(int B, int H, int W, const float* __restrict__ G, const bf16* __rest
             }
 }
 
-// sum of per-CTA partials in CTA order -> dW in (co, ci, dy, dx) layout
-__global__ void k_wgrad_mid_reduce(int nparts, const float* __restrict__ part, float* __restrict__ dw)
+__device__ __forceinline__ float sum_parts(int nparts, size_t stride, const float* __restrict__ p, float (*sl)[33]);
+
+// sum of per-CTA partials (slices of the CTA order) -> dW in (co, ci, dy, dx) layout
+__global__ void __launch_bounds__(1024) k_wgrad_mid_reduce(int nparts, const float* __restrict__ part,
+                                                          float* __restrict__ dw)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;   // index in [co][tap*32 + ci]
-    if (i >= kMidParams) return;
-    float s = 0.f;
-    for (int p = 0; p < nparts; p++) s += part[(size_t)p * kMidParams + i];
-    int co = i / 288, k = i % 288, tap = k / 32, ci = k % 32;
-    dw[(co * kC + ci) * 9 + tap] = s;
+    __shared__ float sl[32][33];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);       // index in [co][tap*32 + ci]
+    const float s = sum_parts(nparts, kMidParams, part + i, sl);
+    const int co = i / 288, k = i % 288, tap = k / 32, ci = k % 32;
+    if (threadIdx.x < 32) dw[(co * kC + ci) * 9 + tap] = s;
 }
 
 // first layer 1 -> 32 with ReLU: h1 = relu(sum_tap w1[co][tap] x[p + tap])
@@ -480,58 +482,112 @@ __global__ void k_conv_out_bwd(int B, int H, int W, const float* __restrict__ dy
 
 // weight gradients of the scalar-channel layers, per-CTA partials (32 x 9):
 // MODE 0: dW1[co][tap] = sum_p g1[p][co] x[p + tap]
-// MODE 1: dW6[ci][tap] = sum_p dy[p] h5[p + tap][ci]
+// MODE 1: dW6[ci][tap] = sum_p dy[p] h5[p + tap][ci] = sum_q h5[q][ci] dy[q - tap]
+// Both are one contraction: a channel image (FP32 g1 or BF16 h5) against the
+// 3 x 3 window of a scalar image.  Lane = channel: a warp takes a run of
+// kWeSeg pixels of one row, so its channel loads are whole 128- (64-) byte
+// pixels, each read once, and the nine products of a pixel read a window that
+// slides along the run (three broadcast words of shared memory per pixel).
+// Bound by the FP32 issue (9 FMA and ~5 loads per pixel and warp) and by the
+// channel image's bytes; one thread per pixel with 288 accumulators re-read
+// the channel image nine times from L1 and ran 650 / 514 us (MODE 0 / 1) at
+// 16 x 128 x 128 pixels, against 12.5 / 13.5 us here (33.5 / 16.8 MB read cold).
+constexpr int kWeSeg = 32;
 template <int MODE>
-__global__ void k_wgrad_edge(int B, int H, int W, const float* __restrict__ gc, const float* __restrict__ xs,
-                             const bf16* __restrict__ hc, float* __restrict__ part)
+__global__ void __launch_bounds__(256)
+k_wgrad_edge(int B, int H, int W, const float* __restrict__ gc, const float* __restrict__ xs,
+             const bf16* __restrict__ hc, float* __restrict__ part)
 {
-    float acc[kC * 9];
+    __shared__ float win[8][3][kWeSeg + 2];         // a warp's scalars: columns sx - 1 .. sx + kWeSeg
+    __shared__ float red[8][kC * 9];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int segs = (W + kWeSeg - 1) / kWeSeg, items = B * H * segs;
+    float acc[9];
 #pragma unroll
-    for (int i = 0; i < kC * 9; i++) acc[i] = 0.f;
-    const size_t npx = (size_t)B * H * W;
-    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += (size_t)gridDim.x * blockDim.x) {
-        const int xx = (int)(p % W), yy = (int)((p / W) % H);
-        const size_t bb = p / ((size_t)H * W);
+    for (int t = 0; t < 9; t++) acc[t] = 0.f;
+    for (int it = blockIdx.x * 8 + w; it < items; it += gridDim.x * 8) {
+        const int row = it / segs, sx = (it - row * segs) * kWeSeg, yy = row % H;
+        const int cnt = min(kWeSeg, W - sx);
+        __syncwarp();
 #pragma unroll
-        for (int tap = 0; tap < 9; tap++) {
-            int gy = yy + tap / 3 - 1, gx = xx + tap % 3 - 1;
-            if (gy < 0 || gy >= H || gx < 0 || gx >= W) continue;
-            size_t q = (bb * H + gy) * W + gx;
-            if (MODE == 0) {
-                float xv = xs[q];
+        for (int r = 0; r < 3; r++) {
+            const bool okr = yy + r - 1 >= 0 && yy + r - 1 < H;
+            const float* sp = xs + (ptrdiff_t)(row + r - 1) * W;
+            for (int c = lane; c < kWeSeg + 2; c += 32) {
+                const int x = sx - 1 + c;
+                win[w][r][c] = okr && x >= 0 && x < W ? __ldg(sp + x) : 0.f;
+            }
+        }
+        __syncwarp();
+        const size_t p0 = ((size_t)row * W + sx) * kC + lane;
+        float s[3][3];
 #pragma unroll
-                for (int c = 0; c < kC; c++) acc[c * 9 + tap] += gc[p * kC + c] * xv;
-            } else {
-                float gv = xs[p];
+        for (int r = 0; r < 3; r++) {
+            s[r][0] = win[w][r][0];
+            s[r][1] = win[w][r][1];
+        }
 #pragma unroll
-                for (int c = 0; c < kC; c++) acc[c * 9 + tap] += gv * __bfloat162float(hc[q * kC + c]);
+        for (int i0 = 0; i0 < kWeSeg; i0 += 8) {
+            if (i0 >= cnt) break;
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const size_t p = p0 + (size_t)(i0 + u) * kC;
+                v[u] = i0 + u < cnt ? (MODE == 0 ? __ldg(gc + p) : __bfloat162float(hc[p])) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+#pragma unroll
+                for (int r = 0; r < 3; r++) s[r][2] = win[w][r][i0 + u + 2];
+#pragma unroll
+                for (int t = 0; t < 9; t++) acc[t] += v[u] * s[t / 3][t % 3];
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    s[r][0] = s[r][1];
+                    s[r][1] = s[r][2];
+                }
             }
         }
     }
-    // block reduction (fixed order) of the 288 accumulators
-    __shared__ float sh[kC * 9];
-    for (int i = threadIdx.x; i < kC * 9; i += blockDim.x) sh[i] = 0.f;
+    // the CTA's eight warps in order; the window of MODE 1 runs against the tap
+#pragma unroll
+    for (int t = 0; t < 9; t++) red[w][lane * 9 + (MODE == 0 ? t : 8 - t)] = acc[t];
     __syncthreads();
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-        if ((int)(threadIdx.x >> 5) == w) {
+    for (int i = threadIdx.x; i < kC * 9; i += 256) {
+        float sum = 0.f;
 #pragma unroll
-            for (int i = 0; i < kC * 9; i++) {
-                float v = warp_sum(acc[i]);
-                if ((threadIdx.x & 31) == 0) sh[i] += v;
-            }
-        }
-        __syncthreads();
+        for (int k = 0; k < 8; k++) sum += red[k][i];
+        part[(size_t)blockIdx.x * kC * 9 + i] = sum;
     }
-    for (int i = threadIdx.x; i < kC * 9; i += blockDim.x) part[(size_t)blockIdx.x * kC * 9 + i] = sh[i];
 }
 
-__global__ void k_wgrad_edge_reduce(int nparts, const float* __restrict__ part, float* __restrict__ dw)
+// One output per lane, the partials in 32 interleaved slices (one per warp)
+// added slice by slice: 32 chains of nparts / 32 loads instead of one of nparts.
+__device__ __forceinline__ float sum_parts(int nparts, size_t stride, const float* __restrict__ p, float (*sl)[33])
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kC * 9) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float s = 0.f;
-    for (int p = 0; p < nparts; p++) s += part[(size_t)p * kC * 9 + i];
-    dw[i] = s;
+    for (int k = w; k < nparts; k += 4 * nw) {      // four loads in flight
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = k + u * nw < nparts ? __ldg(p + (size_t)(k + u * nw) * stride) : 0.f;
+        s += (v[0] + v[1]) + (v[2] + v[3]);
+    }
+    sl[w][lane] = s;
+    __syncthreads();
+    float t = 0.f;
+    if (w == 0)
+        for (int k = 0; k < nw; k++) t += sl[k][lane];
+    return t;                                       // valid in warp 0
+}
+
+__global__ void __launch_bounds__(1024) k_wgrad_edge_reduce(int nparts, const float* __restrict__ part,
+                                                            float* __restrict__ dw)
+{
+    __shared__ float sl[32][33];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);       // 9 CTAs of 32 outputs
+    const float s = sum_parts(nparts, kC * 9, part + i, sl);
+    if (threadIdx.x < 32) dw[i] = s;
 }
 
 // g = d * (a > 0), and g16 = the same in BF16 when given (the TMA input of
@@ -617,7 +673,7 @@ struct jfg_cnn {
 namespace jfg {
 namespace {
 
-constexpr int kEdgeCtas = 296;
+constexpr int kEdgeCtas = 592;                // four CTAs of k_wgrad_edge per SM
 constexpr int kMidWgradCtas = 296;
 
 void cnn_reserve(jfg_cnn* n, size_t npx)
@@ -691,7 +747,7 @@ void wgrad_mid(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float* G,
         ctas = std::min(ntiles, kMidWgradCtas);
         k_wgrad_mid<<<ctas, 288, 0, st>>>(B, H, W, G, X, n->part.p);
     }
-    k_wgrad_mid_reduce<<<(kMidParams + 255) / 256, 256, 0, st>>>(ctas, n->part.p, dw);
+    k_wgrad_mid_reduce<<<kMidParams / 32, 1024, 0, st>>>(ctas, n->part.p, dw);
     JFG_CUDA(cudaGetLastError());
     note_launch(2);
 }
@@ -743,6 +799,13 @@ void cnn_forward(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float* 
     note_launch(2);
 }
 
+// CTAs of k_wgrad_edge: eight runs of kWeSeg pixels each, at most kEdgeCtas
+int edge_ctas(int B, int H, int W)
+{
+    const long long items = (long long)B * H * ((W + kWeSeg - 1) / kWeSeg);
+    return (int)std::min<long long>(kEdgeCtas, (items + 7) / 8);
+}
+
 // gradients of mean((y - t)^2) into n->g32 (forward activations must be current)
 void cnn_backward(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float* x, const float* t)
 {
@@ -753,8 +816,9 @@ void cnn_backward(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float*
     Scratch sc{n->partials.p, n->counter.p};
     vec_launch<1>(st, (int)npx, VLoss{n->y.p, t, n->dy.p, (float)(2.0 / npx)}, sc, nullptr,
                   FinLoss{n->loss.p, 1.0 / npx});
-    k_wgrad_edge<1><<<kEdgeCtas, 256, 0, st>>>(B, H, W, nullptr, n->dy.p, n->h5.p, n->part.p);
-    k_wgrad_edge_reduce<<<2, 256, 0, st>>>(kEdgeCtas, n->part.p, g + kLayerOff[5]);
+    const int ectas = edge_ctas(B, H, W);
+    k_wgrad_edge<1><<<ectas, 256, 0, st>>>(B, H, W, nullptr, n->dy.p, n->h5.p, n->part.p);
+    k_wgrad_edge_reduce<<<9, 1024, 0, st>>>(ectas, n->part.p, g + kLayerOff[5]);
     k_conv_out_bwd<<<grid1d(npx), 256, 0, st>>>(B, H, W, n->dy.p, n->w32.p + kLayerOff[5], n->gA.p);
     // input gradients on the tensor cores (BF16 copies of the gradient images
     // as their TMA inputs) unless JFEM_CNN_TC=0 selects the mma.sync kernels;
@@ -790,8 +854,8 @@ void cnn_backward(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float*
         conv_mid<float, float, 2, false, false>(st, B, H, W, n->gC.p, wt + 0 * kMidParams, n->gB.p, nullptr,
                                                 n->gA.p);                                           // dh1
     k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h1.p, n->gB.p, nullptr);   // g1
-    k_wgrad_edge<0><<<kEdgeCtas, 256, 0, st>>>(B, H, W, n->gB.p, x, nullptr, n->part.p);
-    k_wgrad_edge_reduce<<<2, 256, 0, st>>>(kEdgeCtas, n->part.p, g + kLayerOff[0]);
+    k_wgrad_edge<0><<<ectas, 256, 0, st>>>(B, H, W, n->gB.p, x, nullptr, n->part.p);
+    k_wgrad_edge_reduce<<<9, 1024, 0, st>>>(ectas, n->part.p, g + kLayerOff[0]);
     JFG_CUDA(cudaGetLastError());
     note_launch(9);
 }
