@@ -19,13 +19,14 @@
 //    the halo (start, LBO = plane, SBO = halo row), nothing is copied;
 //  - the weights W[co][k] at (co / 8) * 4608 + (k / 8) * 128 + (co % 8) * 16
 //    + (k % 8) * 2 (LBO = 128, SBO = 4608).
-// Two stages, software-pipelined: the TMA loads of a CTA's tiles run two
+// One accumulator per tap column dx, added in order in the epilogue (as
+// k_conv_ws).  Two stages, software-pipelined: the TMA loads of a CTA's tiles run two
 // tiles ahead and the MMAs of tile i + 1 run while tile i's epilogue reads
-// its own TMEM accumulator (2 x 32 columns).  One thread issues the TMA loads
+// its own TMEM accumulators (2 x 96 columns).  One thread issues the TMA loads
 // and the 18 MMAs (committed to an mbarrier); after the bounded wait each warp reads its
 // 32 TMEM lanes (one pixel per thread, 32 FP32 channels), adds the skip
 // input, applies ReLU and stores BF16.  Persistent CTAs of 128 threads stride
-// over the tiles (~42 KB of shared memory and 64 TMEM columns each).
+// over the tiles (~42 KB of shared memory and 256 TMEM columns each).
 #include <cudaTypedefs.h>
 
 #include "jfg_ops.cuh"
@@ -44,7 +45,7 @@ constexpr int kStages = 2;
 constexpr int kWRowGroup = 36 * 128;             // bytes per 8 output channels (4608)
 constexpr int kWBytes = 4 * kWRowGroup;          // 18,432
 constexpr int kTcThreads = 128;
-constexpr int kTcCtasPerSm = 5;
+constexpr int kTcCtasPerSm = 2;                  // 256 TMEM columns each
 // kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major, N = 32, M = 128
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
 
@@ -92,76 +93,94 @@ __device__ __forceinline__ void tma_plane(uint32_t dst, const CUtensorMap* map, 
 //             (an input gradient through the next layer's ReLU, and its BF16
 //             copy: the TMA input of the following input-gradient convolution)
 //   kBwdSkip: out(f32) = acc + skip(f32)                     input gradient plus the skip path's
-constexpr int kFwd = 0, kFwdSkip = 1, kBwdMask = 2, kBwdSkip = 3;
 //   kFwdProj: the last 32 -> 32 layer (with skip) fused with the projection of
 //   the 32 -> 1 output layer: h = relu(acc + skip) rounded to BF16 (the values
 //   the output layer would read back), then u[t][p] = sum_c w6[c][t] h[c] for
 //   the nine taps t, written as nine FP32 planes; y = sum_t u[t][p + off_t]
 //   follows in a small kernel.  Warp-specialised kernel only.
-constexpr int kFwdProj = 4;
+constexpr int kFwd = 0, kFwdSkip = 1, kBwdMask = 2, kBwdSkip = 3, kFwdProj = 4;
 
-// The epilogue of one output pixel: its 32 FP32 channel sums r (from TMEM)
-// combined and stored as MODE says; base = the pixel's first channel.
+// The image a mode's epilogue reads beside the accumulator, one pixel: 32
+// BF16 (skip or mask) or 32 FP32 (skip) channels.
 template <int MODE>
-__device__ __forceinline__ void conv_store(const uint32_t (&r)[32], size_t base, const void* __restrict__ aux,
-                                           void* __restrict__ out, bf16* __restrict__ out16)
+struct AuxPx {
+    static constexpr int kVecs = MODE == kFwd ? 0 : (MODE == kBwdSkip ? 8 : 4);
+    uint4 q[kVecs ? kVecs : 1];
+    __device__ __forceinline__ void load(const void* __restrict__ aux, size_t pix, bool inside)
+    {
+#pragma unroll
+        for (int i = 0; i < kVecs; i++)
+            q[i] = inside ? __ldg(reinterpret_cast<const uint4*>(aux) + pix * kVecs + i) : make_uint4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ float at(int c) const      // channel c
+    {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(q);
+        if (MODE == kBwdSkip) return __uint_as_float(w[c]);
+        const uint32_t u = w[c >> 1];
+        return __uint_as_float(c & 1 ? u & 0xFFFF0000u : u << 16);
+    }
+};
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
-    if constexpr (MODE == kFwd || MODE == kFwdSkip) {
-        __align__(16) bf16 o[32];
-        __align__(16) bf16 sv[32];
-        if (MODE == kFwdSkip) {
-            const bf16* skip = static_cast<const bf16*>(aux);
+    const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+// 32 bytes (one sector) per thread in one store; p 32-byte aligned
+__device__ __forceinline__ void st_sector(void* p, const uint32_t (&w)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+// Channels c0 .. c0 + 15 of one output pixel: the sums v combined with the
+// pixel's aux image and stored as MODE says (not kFwdProj).
+template <int MODE>
+__device__ __forceinline__ void conv_emit(const float (&v)[16], int c0, const AuxPx<MODE>& aux, size_t pix,
+                                          void* __restrict__ out, bf16* __restrict__ out16)
+{
+    float f[16];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                *reinterpret_cast<uint4*>(sv + 8 * q) =
-                    __ldg(reinterpret_cast<const uint4*>(skip + base + 8 * q));
-        }
+    for (int c = 0; c < 16; c++) {
+        if (MODE == kFwd) f[c] = fmaxf(v[c], 0.f);
+        if (MODE == kFwdSkip) f[c] = fmaxf(v[c] + aux.at(c0 + c), 0.f);
+        if (MODE == kBwdMask) f[c] = aux.at(c0 + c) > 0.f ? v[c] : 0.f;
+        if (MODE == kBwdSkip) f[c] = v[c] + aux.at(c0 + c);
+    }
+    const size_t base = pix * 32 + c0;
+    if (MODE == kBwdMask || MODE == kBwdSkip) {
+        float* of = static_cast<float*>(out) + base;
 #pragma unroll
-        for (int c = 0; c < 32; c++) {
-            float v = __uint_as_float(r[c]);
-            if (MODE == kFwdSkip) v += __bfloat162float(sv[c]);
-            o[c] = __float2bfloat16_rn(fmaxf(v, 0.f));
-        }
-        bf16* ob = static_cast<bf16*>(out);
+        for (int h = 0; h < 2; h++) {
+            uint32_t w[8];
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-            *reinterpret_cast<uint4*>(ob + base + 8 * q) = *reinterpret_cast<const uint4*>(o + 8 * q);
-    } else if constexpr (MODE == kBwdMask) {
-        const bf16* mask = static_cast<const bf16*>(aux);
-        __align__(16) bf16 mv[32];
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            *reinterpret_cast<uint4*>(mv + 8 * q) = __ldg(reinterpret_cast<const uint4*>(mask + base + 8 * q));
-        __align__(16) float f[32];
-        __align__(16) bf16 o[32];
-#pragma unroll
-        for (int c = 0; c < 32; c++) {
-            const float v = __bfloat162float(mv[c]) > 0.f ? __uint_as_float(r[c]) : 0.f;
-            f[c] = v;
-            o[c] = __float2bfloat16_rn(v);
-        }
-        float* of = static_cast<float*>(out);
-#pragma unroll
-        for (int q = 0; q < 8; q++)
-            *reinterpret_cast<float4*>(of + base + 4 * q) = *reinterpret_cast<const float4*>(f + 4 * q);
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            *reinterpret_cast<uint4*>(out16 + base + 8 * q) = *reinterpret_cast<const uint4*>(o + 8 * q);
-    } else {
-        const float* skip = static_cast<const float*>(aux);
-        float* of = static_cast<float*>(out);
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const float4 sk = __ldg(reinterpret_cast<const float4*>(skip + base + 4 * q));
-            float4 v;
-            v.x = __uint_as_float(r[4 * q]) + sk.x;
-            v.y = __uint_as_float(r[4 * q + 1]) + sk.y;
-            v.z = __uint_as_float(r[4 * q + 2]) + sk.z;
-            v.w = __uint_as_float(r[4 * q + 3]) + sk.w;
-            *reinterpret_cast<float4*>(of + base + 4 * q) = v;
+            for (int c = 0; c < 8; c++) w[c] = __float_as_uint(f[8 * h + c]);
+            st_sector(of + 8 * h, w);
         }
     }
+    if (MODE != kBwdSkip) {
+        uint32_t w[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) w[c] = pack_bf16(f[2 * c], f[2 * c + 1]);
+        st_sector((MODE == kBwdMask ? out16 : static_cast<bf16*>(out)) + base, w);
+    }
 }
+
+// 16 consecutive TMEM columns of this warp's 32 lanes
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16])
+{
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+#pragma unroll
+    for (int c = 0; c < 16; c++) v[c] = __uint_as_float(r[c]);
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads)
@@ -180,7 +199,7 @@ k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, cons
         *reinterpret_cast<uint4*>(wsm + (co >> 3) * kWRowGroup + j * 128 + (co & 7) * 16) = v;
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(&tmem_sh))
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(&tmem_sh))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -229,12 +248,12 @@ k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, cons
             for (int k = 0; k < 2; k++) {
                 const uint64_t da = umma_desc(hb + 2 * k * kPlane + (dy * kHW + dx) * 16, kPlane, kHW * 16);
                 const uint64_t db = umma_desc(wbase + (4 * tap + 2 * k) * 128, 128, kWRowGroup);
-                const uint32_t accum = (tap | k) ? 1u : 0u;
+                const uint32_t accum = (dy | k) ? 1u : 0u;     // one accumulator per tap column dx
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                    ::"r"(tmem + (uint32_t)(s * 32)), "l"(da), "l"(db), "r"(kIdesc), "r"(accum)
+                    ::"r"(tmem + (uint32_t)(s * 128 + dx * 32)), "l"(da), "l"(db), "r"(kIdesc), "r"(accum)
                     : "memory");
             }
         }
@@ -286,27 +305,26 @@ k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, cons
             }
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint32_t r[32];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-              "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-              "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-              "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(s * 32))
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int t = tile_of(i);
         const int b = t / per_img, rem = t - b * per_img;
         const int y0 = (rem / tilesx) * kTH, x0 = (rem % tilesx) * kTW;
         const int m = warp * 32 + lane;
         const int gy = y0 + (m >> 3), gx = x0 + (m & 7);
-        if (gy < H && gx < W) {
-            const size_t base = (((size_t)b * H + gy) * W + gx) * 32;
-            conv_store<MODE>(r, base, aux, out, out16);
+        const bool inside = gy < H && gx < W;
+        const size_t pix = inside ? ((size_t)b * H + gy) * W + gx : 0;
+        AuxPx<MODE> ax;
+        ax.load(aux, pix, inside);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(s * 128 + 16 * h);
+            float d0[16], d1[16], d2[16];
+            tmem_ld16(col, d0);
+            tmem_ld16(col + 32, d1);
+            tmem_ld16(col + 64, d2);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 16; c++) d0[c] = (d0[c] + d1[c]) + d2[c];
+            if (inside) conv_emit<MODE>(d0, 16 * h, ax, pix, out, out16);
         }
         // every thread's TMEM reads are done before the MMAs two tiles on overwrite this stage
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -322,64 +340,57 @@ k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, cons
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
     }
 }
 
 // ---------------------------------------------------------------------------
-// Warp-specialised pipeline (the default).  Per CTA of 256 threads:
-//   warp 0 (one lane): TMA producer -- tile i's whole halo (18 x 10 pixels x
-//     32 channels) as ONE box with a 64-byte inner extent into staging buffer
-//     i % ST, once the transposers released it (mbarrier `sempty`); one
-//     64-byte row per pixel instead of four 16-byte ones;
-//   warps 6-7: transposers -- wait for the box (`sfull`, transaction bytes)
-//     and for a free plane buffer (`pempty`), copy the pixels' four 16-byte
-//     channel chunks into the four 8-channel planes the MMA descriptors view,
-//     make those writes visible to the tensor core (fence.proxy.async) and
-//     release the staging buffer (`sempty`) and publish the planes (`pfull`);
-//   warp 1 (one lane): MMA issuer -- waits for the planes (`pfull`) and a free
-//     TMEM accumulator (`tempty`), issues the 18 MMAs and commits them to
-//     `pempty` (planes free) and `tfull` (accumulator ready);
-//   warps 2-5: epilogue -- each reads its 32 TMEM lanes (warp w owns lanes
-//     32 (w % 4) ...) of the ready accumulator, releases it (`tempty`, one
-//     arrival per warp), then combines and stores its 32 pixels.
+// Warp-specialised pipeline (the default).
+//
+// The three taps of a row are one MMA: for an input pixel q the products with
+// the weights of dx = 0, 1, 2 (N = 3 x 32 outputs) go to three accumulators
+// D_dx[q], summed over dy and the channels, and the output is
+//   out[p] = (D_0[p - 1] + D_1[p]) + D_2[p + 1].
+// A tile is kRY rows of kRX = 32 input pixels (M = 128, TMEM lane = row, x), so
+// the lanes of an epilogue warp are one row's consecutive pixels, the shifts
+// are two shuffles inside the warp and 30 of its 32 pixels are outputs.  The
+// input arrives as ONE TMA box (32 channels x 32 pixels x kRY + 2 rows,
+// 64-byte swizzle) which is the K-major A operand as it lies: tap row dy is
+// dy * 2,048 bytes further.  6 MMAs of N = 96 per tile of 120 outputs instead
+// of 18 of N = 32 per 128: each MMA of N = 32 held the tensor pipe ~40 cycles
+// for 16 cycles of math, and the kernel that fed them from transposed 8-channel
+// planes (shared memory read and written once more per tile) ran 55 us per
+// layer at 1025 x 1025 pixels against 32.5 us here (63 -> 41.5 us with a skip
+// input, 86 -> 65 us with the output projection); the image bytes (134 MB) take
+// 20 us.
+//
+// Roles (320 threads, two CTAs per SM, 256 TMEM columns each):
+//   warp 0 (one lane): TMA producer, kDxStages boxes ahead (`full` / `empty`);
+//   warp 1 (one lane): MMA issuer -- waits for a box and a free accumulator
+//     set (`tempty`), issues the 6 MMAs and commits them to `empty` and `tfull`;
+//   warps 2-9: epilogue, two groups of four taking the tiles in turn (group =
+//     accumulator set); a warp loads its pixels' aux channels before it waits.
 // No CTA-wide barrier inside the tile loop.  Every wait is bounded
 // (mbar_wait); a timeout sets *err, every role stops, and the copies and MMAs
 // still in flight are waited for (bounded) before TMEM is released.
-constexpr int kWsAcc = 2;
-constexpr int kWsThreads = 256;
-constexpr int kStageBytes = kHH * kHW * 64;      // 11,520: the halo as 64-byte pixels
-// shared memory of a CTA with ST stages (+ alignment slack); CTAs per SM as
-// many as fit 228 KB, at most 8 (64 TMEM columns each)
-template <int ST> constexpr int ws_smem() { return kWBytes + ST * (kStageBytes + kHaloBytes) + 128; }
-template <int ST> constexpr int ws_ctas_per_sm() { return 228 * 1024 / (ws_smem<ST>() + 1024) < 8 ? 228 * 1024 / (ws_smem<ST>() + 1024) : 8; }
+// ---------------------------------------------------------------------------
+constexpr int kRX = 32, kRY = 4;                 // input pixels of a tile: 4 rows of 32
+constexpr int kOutX = kRX - 2;                   // output pixels of a tile row
+constexpr int kBoxRows = kRY + 2;
+constexpr int kRowBytes = kRX * 64;              // one input row of the box
+constexpr int kBoxBytes = kBoxRows * kRowBytes;  // 12,288
+constexpr int kDxStages = 4;
+constexpr int kDxAcc = 2;                        // accumulator sets of 96 columns, 128 apart
+constexpr int kDxThreads = 320;
+constexpr int kDxCtasPerSm = 2;
+constexpr int kDxWGroup = 12 * 128;              // weights: bytes per 8 rows n = dx * 32 + co (k = dy * 32 + ci)
+constexpr int kDxSmem = kDxStages * kBoxBytes + 12 * kDxWGroup + 1024;
+constexpr uint32_t kIdesc96 = (1u << 4) | (1u << 7) | (1u << 10) | ((96u >> 3) << 17) | ((128u >> 4) << 24);
 
-// kFwdProj epilogue of one pixel (see kFwdProj); w6s is [tap][channel] FP32
-__device__ __forceinline__ void proj_store(const uint32_t (&r)[32], size_t pix, size_t npx,
-                                           const bf16* __restrict__ skip, const float* w6s, float* __restrict__ u)
+// K-major operand rows of 64 bytes, 64-byte swizzle (8-row groups 512 bytes apart)
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr)
 {
-    __align__(16) bf16 sv[32];
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-        *reinterpret_cast<uint4*>(sv + 8 * q) = __ldg(reinterpret_cast<const uint4*>(skip + pix * 32 + 8 * q));
-    float h[32];
-#pragma unroll
-    for (int c = 0; c < 32; c++)
-        h[c] = __bfloat162float(__float2bfloat16_rn(fmaxf(__uint_as_float(r[c]) + __bfloat162float(sv[c]), 0.f)));
-#pragma unroll
-    for (int t = 0; t < 9; t++) {
-        const float4* w4 = reinterpret_cast<const float4*>(w6s + t * 32);
-        float acc = 0.f;
-#pragma unroll
-        for (int c4 = 0; c4 < 8; c4++) {
-            const float4 w = w4[c4];
-            acc += w.x * h[4 * c4];
-            acc += w.y * h[4 * c4 + 1];
-            acc += w.z * h[4 * c4 + 2];
-            acc += w.w * h[4 * c4 + 3];
-        }
-        u[(size_t)t * npx + pix] = acc;
-    }
+    return umma_desc(saddr, 16, 512) | ((uint64_t)4 << 61);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
@@ -387,47 +398,43 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-template <int MODE, int ST>
-__global__ void __launch_bounds__(kWsThreads)
+template <int MODE>
+__global__ void __launch_bounds__(kDxThreads, kDxCtasPerSm)
 k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf16* __restrict__ wk,
           const void* __restrict__ aux, void* __restrict__ out, bf16* __restrict__ out16, int* __restrict__ err,
           const float* __restrict__ proj)
 {
     extern __shared__ unsigned char dsm_raw[];
-    unsigned char* dsm = reinterpret_cast<unsigned char*>(((uintptr_t)dsm_raw + 127) & ~(uintptr_t)127);
-    unsigned char* wsm = dsm;                                 // weights, kWBytes
-    unsigned char* stage = dsm + kWBytes;                     // ST x kStageBytes (TMA boxes)
-    unsigned char* planes = stage + ST * kStageBytes;         // ST x kHaloBytes (MMA operands)
-    __shared__ __align__(8) uint64_t sfull[ST], sempty[ST], pfull[ST], pempty[ST], tfull[kWsAcc], tempty[kWsAcc];
+    unsigned char* boxes = reinterpret_cast<unsigned char*>(((uintptr_t)dsm_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* wsm = boxes + kDxStages * kBoxBytes;
+    __shared__ __align__(8) uint64_t full[kDxStages], empty[kDxStages], tfull[kDxAcc], tempty[kDxAcc];
     __shared__ uint32_t tmem_sh;
     __shared__ volatile int s_stop;
-    __shared__ int s_loads, s_trans, s_mmas;                  // progress counts, for the error path
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < 32 * 36; i += kWsThreads) {
-        const int co = i / 36, j = i % 36;
-        const uint4 v = *reinterpret_cast<const uint4*>(wk + co * 288 + j * 8);
-        *reinterpret_cast<uint4*>(wsm + (co >> 3) * kWRowGroup + j * 128 + (co & 7) * 16) = v;
-    }
+    __shared__ int s_loads, s_mmas;                           // progress counts, for the error path
     __shared__ __align__(16) float w6s[MODE == kFwdProj ? 9 * 32 : 4];    // output-layer weights [tap][channel]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int i = tid; i < 32 * 36; i += kDxThreads) {
+        const int co = i / 36, j = i % 36, tap = j >> 2, part = j & 3;
+        const int n = (tap % 3) * 32 + co, kg = (tap / 3) * 4 + part;
+        *reinterpret_cast<uint4*>(wsm + (n >> 3) * kDxWGroup + kg * 128 + (n & 7) * 16) =
+            *reinterpret_cast<const uint4*>(wk + co * 288 + j * 8);
+    }
     if constexpr (MODE == kFwdProj)
-        for (int i = tid; i < 9 * 32; i += kWsThreads) w6s[(i % 9) * 32 + i / 9] = proj[i];
+        for (int i = tid; i < 9 * 32; i += kDxThreads) w6s[(i % 9) * 32 + i / 9] = proj[i];
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(&tmem_sh))
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(&tmem_sh))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 32) {
         s_stop = 0;
         s_loads = 0;
-        s_trans = 0;
         s_mmas = 0;
-        for (int q = 0; q < ST; q++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sfull[q])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(smem_u32(&sempty[q])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(smem_u32(&pfull[q])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&pempty[q])) : "memory");
+        for (int q = 0; q < kDxStages; q++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[q])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[q])) : "memory");
         }
-        for (int q = 0; q < kWsAcc; q++) {
+        for (int q = 0; q < kDxAcc; q++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&tfull[q])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&tempty[q])) : "memory");
         }
@@ -438,8 +445,8 @@ k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_sh;
-    const uint32_t wbase = smem_u32(wsm);
-    const int tilesx = (W + kTW - 1) / kTW, tilesy = (H + kTH - 1) / kTH;
+    const uint32_t wbase = smem_u32(wsm), bbase = smem_u32(boxes);
+    const int tilesx = (W + kOutX - 1) / kOutX, tilesy = (H + kRY - 1) / kRY;
     const int per_img = tilesx * tilesy;
     const int ntiles = per_img * B;
     const int cnt = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -448,79 +455,48 @@ k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf
     if (warp == 0) {
         if (lane == 0) {                               // TMA producer
             for (int i = 0; i < cnt && !s_stop; i++) {
-                const int q = i % ST;
-                if (i >= ST && !mbar_wait(smem_u32(&sempty[q]), (uint32_t)((i / ST - 1) & 1))) {
+                const int q = i % kDxStages;
+                if (i >= kDxStages && !mbar_wait(smem_u32(&empty[q]), (uint32_t)((i / kDxStages - 1) & 1))) {
                     s_stop = 1;
                     break;
                 }
                 const int t = tile_of(i);
                 const int b = t / per_img, rem = t - b * per_img;
-                const int y0 = (rem / tilesx) * kTH, x0 = (rem % tilesx) * kTW;
-                const uint32_t bar = smem_u32(&sfull[q]);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kStageBytes)
+                const int y0 = (rem / tilesx) * kRY, x0 = (rem % tilesx) * kOutX;
+                const uint32_t bar = smem_u32(&full[q]);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kBoxBytes)
                              : "memory");
-                tma_plane(smem_u32(stage + q * kStageBytes), &tin, 0, x0 - 1, y0 - 1, b, bar);
+                tma_plane(bbase + q * kBoxBytes, &tin, 0, x0 - 1, y0 - 1, b, bar);
                 s_loads = i + 1;
-            }
-        }
-    } else if (warp >= 6) {                            // transposers
-        const int tt = tid - 192;
-        for (int i = 0; i < cnt; i++) {
-            const int q = i % ST;
-            bool ok = !s_stop && mbar_wait(smem_u32(&sfull[q]), (uint32_t)((i / ST) & 1));
-            if (ok && i >= ST) ok = mbar_wait(smem_u32(&pempty[q]), (uint32_t)((i / ST - 1) & 1));
-            if (!__all_sync(0xffffffffu, ok)) {
-                if (lane == 0) s_stop = 1;
-                break;
-            }
-            const unsigned char* src = stage + q * kStageBytes;
-            unsigned char* dst = planes + q * kHaloBytes;
-            for (int m = tt; m < kHH * kHW * 4; m += 64) {
-                const int pix = m >> 2, part = m & 3;
-                *reinterpret_cast<uint4*>(dst + part * kPlane + pix * 16) =
-                    *reinterpret_cast<const uint4*>(src + pix * 64 + part * 16);
-            }
-            // the planes are read by the tensor core (async proxy)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(smem_u32(&sempty[q]));
-                mbar_arrive(smem_u32(&pfull[q]));
-                if (warp == 6) s_trans = i + 1;
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {                               // MMA issuer
             for (int i = 0; i < cnt && !s_stop; i++) {
-                const int q = i % ST, a = i % kWsAcc;
-                if (!mbar_wait(smem_u32(&pfull[q]), (uint32_t)((i / ST) & 1))) {
-                    s_stop = 1;
-                    break;
-                }
-                if (i >= kWsAcc && !mbar_wait(smem_u32(&tempty[a]), (uint32_t)((i / kWsAcc - 1) & 1))) {
+                const int q = i % kDxStages, a = i % kDxAcc;
+                if (!mbar_wait(smem_u32(&full[q]), (uint32_t)((i / kDxStages) & 1)) ||
+                    (i >= kDxAcc && !mbar_wait(smem_u32(&tempty[a]), (uint32_t)((i / kDxAcc - 1) & 1)))) {
                     s_stop = 1;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t hb = smem_u32(planes + q * kHaloBytes);
 #pragma unroll
-                for (int tap = 0; tap < 9; tap++) {
-                    const int dy = tap / 3, dx = tap % 3;
+                for (int dy = 0; dy < 3; dy++) {
 #pragma unroll
                     for (int k = 0; k < 2; k++) {
-                        const uint64_t da = umma_desc(hb + 2 * k * kPlane + (dy * kHW + dx) * 16, kPlane, kHW * 16);
-                        const uint64_t db = umma_desc(wbase + (4 * tap + 2 * k) * 128, 128, kWRowGroup);
-                        const uint32_t accum = (tap | k) ? 1u : 0u;
+                        const uint64_t da = umma_desc_sw64(bbase + q * kBoxBytes + dy * kRowBytes + k * 32);
+                        const uint64_t db = umma_desc(wbase + (4 * dy + 2 * k) * 128, 128, kDxWGroup);
+                        const uint32_t accum = (dy | k) ? 1u : 0u;
                         asm volatile(
                             "{\n\t.reg .pred p;\n\t"
                             "setp.ne.b32 p, %4, 0;\n\t"
                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                            ::"r"(tmem + (uint32_t)(a * 32)), "l"(da), "l"(db), "r"(kIdesc), "r"(accum)
+                            ::"r"(tmem + (uint32_t)(a * 128)), "l"(da), "l"(db), "r"(kIdesc96), "r"(accum)
                             : "memory");
                     }
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&pempty[q]))
+                                 smem_u32(&empty[q]))
                              : "memory");
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                  smem_u32(&tfull[a]))
@@ -528,43 +504,70 @@ k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf
                 s_mmas = i + 1;
             }
         }
-    } else {                                           // epilogue warps 2..5
-        const int lg = warp & 3;                       // TMEM lane group this warp may access
-        const int m = lg * 32 + lane;                  // pixel of the 16 x 8 tile
-        for (int i = 0; i < cnt; i++) {
-            const int a = i % kWsAcc;
-            const bool ok = !s_stop && mbar_wait(smem_u32(&tfull[a]), (uint32_t)((i / kWsAcc) & 1));
+    } else {                                           // epilogue warps 2..9
+        const int lg = warp & 3;                       // TMEM lane group this warp may access = tile row
+        for (int i = (warp - 2) >> 2; i < cnt; i += kDxAcc) {
+            const int a = i % kDxAcc;
+            const int t = tile_of(i);
+            const int b = t / per_img, rem = t - b * per_img;
+            const int gy = (rem / tilesx) * kRY + lg, gx = (rem % tilesx) * kOutX + lane - 1;
+            const bool inside = gy < H && gx < W && lane >= 1 && lane <= kOutX;
+            const size_t pix = inside ? ((size_t)b * H + gy) * W + gx : 0;
+            AuxPx<MODE> ax;
+            ax.load(aux, pix, inside);
+            const bool ok = !s_stop && mbar_wait(smem_u32(&tfull[a]), (uint32_t)((i / kDxAcc) & 1));
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) s_stop = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t r[32];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                : "r"(tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)(a * 32))
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&tempty[a]));
-            const int t = tile_of(i);
-            const int b = t / per_img, rem = t - b * per_img;
-            const int gy = (rem / tilesx) * kTH + (m >> 3), gx = (rem % tilesx) * kTW + (m & 7);
-            if (gy < H && gx < W) {
-                const size_t pix = ((size_t)b * H + gy) * W + gx;
-                if constexpr (MODE == kFwdProj)
-                    proj_store(r, pix, (size_t)B * H * W, static_cast<const bf16*>(aux), w6s,
-                               static_cast<float*>(out));
-                else
-                    conv_store<MODE>(r, pix * 32, aux, out, out16);
+            float u9[9];
+            if constexpr (MODE == kFwdProj) {
+#pragma unroll
+                for (int tp = 0; tp < 9; tp++) u9[tp] = 0.f;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t col = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)(a * 128 + 16 * h);
+                float d0[16], d1[16], d2[16];
+                tmem_ld16(col, d0);
+                tmem_ld16(col + 32, d1);
+                tmem_ld16(col + 64, d2);
+                tmem_ld_wait();
+                if (h == 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&tempty[a]));
+                }
+#pragma unroll
+                for (int c = 0; c < 16; c++)
+                    d0[c] = (__shfl_up_sync(0xffffffffu, d0[c], 1) + d1[c]) + __shfl_down_sync(0xffffffffu, d2[c], 1);
+                if constexpr (MODE == kFwdProj) {
+#pragma unroll
+                    for (int c = 0; c < 16; c++)
+                        d0[c] = __bfloat162float(__float2bfloat16_rn(fmaxf(d0[c] + ax.at(16 * h + c), 0.f)));
+#pragma unroll
+                    for (int tp = 0; tp < 9; tp++) {
+                        const float4* w4 = reinterpret_cast<const float4*>(w6s + tp * 32 + 16 * h);
+#pragma unroll
+                        for (int c4 = 0; c4 < 4; c4++) {
+                            const float4 w = w4[c4];
+                            u9[tp] += w.x * d0[4 * c4];
+                            u9[tp] += w.y * d0[4 * c4 + 1];
+                            u9[tp] += w.z * d0[4 * c4 + 2];
+                            u9[tp] += w.w * d0[4 * c4 + 3];
+                        }
+                    }
+                } else {
+                    if (inside) conv_emit<MODE>(d0, 16 * h, ax, pix, out, out16);
+                }
+            }
+            if constexpr (MODE == kFwdProj) {
+                float* u = static_cast<float*>(out);
+                const size_t npx = (size_t)B * H * W;
+                if (inside)
+#pragma unroll
+                    for (int tp = 0; tp < 9; tp++) u[(size_t)tp * npx + pix] = u9[tp];
             }
         }
     }
@@ -572,300 +575,15 @@ k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf
     if (s_stop && tid == 32) {
         // report, then let the copies and MMAs still in flight finish (bounded) before TMEM is freed
         atomicOr(err, 1);
-        const int nl = s_loads, nt = s_trans, nm = s_mmas;
-        for (int k = nt; k < nl; k++) mbar_wait(smem_u32(&sfull[k % ST]), (uint32_t)((k / ST) & 1));
-        if (nm > 0) mbar_wait(smem_u32(&tfull[(nm - 1) % kWsAcc]), (uint32_t)(((nm - 1) / kWsAcc) & 1));
+        const int nl = s_loads, nm = s_mmas;
+        for (int k = nm; k < nl; k++) mbar_wait(smem_u32(&full[k % kDxStages]), (uint32_t)((k / kDxStages) & 1));
+        if (nm > 0) mbar_wait(smem_u32(&tfull[(nm - 1) % kDxAcc]), (uint32_t)(((nm - 1) / kDxAcc) & 1));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Strip convolution: the activations are the MMA's A operand in TMEM.
-//
-// A work item is a strip of 128 consecutive output pixels of a row (the
-// MMA's M: TMEM lane = x position) over a segment of rows.  Each input row
-// (130 pixels with the x halo) arrives in shared memory by four TMA boxes of
-// 8 channels (the canonical K-major planes of the tiled kernels), and one
-// thread copies it into TMEM three times, shifted by -1, 0, +1 pixels
-// (tcgen05.cp 128x256b: 128 lanes x 16 channels per copy), so that the tap
-// (dy, dx) of output row y reads input row y + dy - 1 at its dx copy.  The 18
-// MMAs of an output row (9 taps x K = 16 twice, N = 32) then read only the
-// weights from shared memory: 1 KB per MMA instead of 4 KB of A plus 1 KB of
-// B.  Rows live in a ring of four TMEM slots (48 columns each: 3 shifts x
-// 16); two 32-column accumulators let the epilogue of row j overlap the MMAs
-// of row j + 1; 256 TMEM columns per CTA, two CTAs per SM.  The MMAs of every output pixel run in the tiled kernels'
-// order (taps in order, two K halves), so the results are theirs bit for
-// bit.  Roles: warp 0 TMA producer, warp 1 copy + MMA issuer, warps 2-5
-// epilogue (conv_store / proj_store of the tiled kernels).  Every wait is
-// bounded; a timeout sets *err and the CTA drains what it issued.
-// ---------------------------------------------------------------------------
-constexpr int kSW = 128;                         // output pixels of a strip row (M)
-constexpr int kSPx = kSW + 2;                    // input pixels of a row, x halo included
-constexpr int kSPlane = 2176;                    // plane stride: 130 x 16 B rounded up to 128
-constexpr int kSRowBytes = 4 * kSPlane;          // one input row in four 8-channel planes
-constexpr int kSRows = 6;                        // input rows in shared memory
-constexpr int kSSlots = 4;                       // input rows in TMEM
-constexpr int kSSlotCols = 48;                   // TMEM columns of a row: 3 shifts x 16
-constexpr int kSDcol = kSSlots * kSSlotCols;     // TMEM column of the two accumulators (192)
-constexpr int kSTmemCols = 256;
-constexpr int kSCtasPerSm = 2;
-constexpr int kSThreads = 192;
-// two CTAs per SM (256 TMEM columns each): the request is padded past a third
-// of the SM's shared memory, so that no third CTA (which would wait for TMEM)
-// is placed
-constexpr int kStripSmemUsed = kWBytes + kSRows * kSRowBytes + 128;
-constexpr int kStripSmem = kStripSmemUsed > 80 * 1024 ? kStripSmemUsed : 80 * 1024;
-
-struct StripGeo {
-    int B, H, W, nstrips, nsegs, rs;            // rs: output rows per segment
-};
-
-__device__ __forceinline__ void strip_item(const StripGeo& g, int t, int& b, int& sx, int& y0, int& y1)
-{
-    const int per_img = g.nstrips * g.nsegs;
-    b = t / per_img;
-    const int rem = t - b * per_img;
-    sx = rem / g.nsegs;
-    y0 = (rem - sx * g.nsegs) * g.rs;
-    y1 = min(g.H, y0 + g.rs);
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kSThreads, kSCtasPerSm)
-k_conv_strip(const __grid_constant__ CUtensorMap trow, StripGeo g, const bf16* __restrict__ wk,
-             const void* __restrict__ aux, void* __restrict__ out, bf16* __restrict__ out16, int* __restrict__ err,
-             const float* __restrict__ proj)
-{
-    extern __shared__ unsigned char dsm_raw[];
-    unsigned char* dsm = reinterpret_cast<unsigned char*>(((uintptr_t)dsm_raw + 127) & ~(uintptr_t)127);
-    unsigned char* wsm = dsm;                                  // weights, kWBytes
-    unsigned char* rows = dsm + kWBytes;                       // kSRows input rows
-    __shared__ __align__(8) uint64_t rfull[kSRows], rcp[kSRows], dfull[2], dempty[2];
-    __shared__ uint32_t tmem_sh;
-    __shared__ volatile int s_stop;
-    __shared__ int s_loads, s_copies, s_mmas;                  // progress counts, for the error path
-    __shared__ __align__(16) float w6s[MODE == kFwdProj ? 9 * 32 : 4];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < 32 * 36; i += kSThreads) {
-        const int co = i / 36, j = i % 36;
-        const uint4 v = *reinterpret_cast<const uint4*>(wk + co * 288 + j * 8);
-        *reinterpret_cast<uint4*>(wsm + (co >> 3) * kWRowGroup + j * 128 + (co & 7) * 16) = v;
-    }
-    if constexpr (MODE == kFwdProj)
-        for (int i = tid; i < 9 * 32; i += kSThreads) w6s[(i % 9) * 32 + i / 9] = proj[i];
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
-                     "n"(kSTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 32) {
-        s_stop = 0;
-        s_loads = 0;
-        s_copies = 0;
-        s_mmas = 0;
-        for (int q = 0; q < kSRows; q++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&rfull[q])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&rcp[q])) : "memory");
-        }
-        for (int q = 0; q < 2; q++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&dfull[q])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&dempty[q])) : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // weights: generic writes, async-proxy reads
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_sh;
-    const uint32_t wbase = smem_u32(wsm);
-    const uint32_t rbase = smem_u32(rows);
-    const int items = g.B * g.nstrips * g.nsegs;
-    const int cnt = (int)blockIdx.x < items ? (items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-
-    if (warp == 0) {
-        if (lane == 0) {                               // TMA producer: the input rows of every item in order
-            int q = 0;
-            for (int i = 0; i < cnt && !s_stop; i++) {
-                int b, sx, y0, y1;
-                strip_item(g, (int)blockIdx.x + i * (int)gridDim.x, b, sx, y0, y1);
-                for (int yin = y0 - 1; yin <= y1 && !s_stop; yin++, q++) {
-                    const int sl = q % kSRows;
-                    if (q >= kSRows && !mbar_wait(smem_u32(&rcp[sl]), (uint32_t)((q / kSRows - 1) & 1))) {
-                        s_stop = 1;
-                        break;
-                    }
-                    const uint32_t bar = smem_u32(&rfull[sl]);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                                 "r"(4 * kSPx * 16)
-                                 : "memory");
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        tma_plane(rbase + sl * kSRowBytes + c * kSPlane, &trow, 8 * c, sx * kSW - 1, yin, b, bar);
-                    s_loads = q + 1;
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            int q = 0;                                 // input rows copied into TMEM (CTA-wide sequence)
-            int j = 0;                                 // output rows issued
-            // input row qq: wait for its TMA boxes, copy it three times shifted
-            // into TMEM slot qq % kSSlots, commit the copies to rcp
-            auto copy_row = [&](int qq) -> bool {
-                const int sl = qq % kSRows;
-                if (!mbar_wait(smem_u32(&rfull[sl]), (uint32_t)((qq / kSRows) & 1))) return false;
-                const uint32_t src = rbase + sl * kSRowBytes;
-                const uint32_t dst = tmem + (uint32_t)((qq % kSSlots) * kSSlotCols);
-#pragma unroll
-                for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                    for (int kh = 0; kh < 2; kh++) {
-                        const uint64_t sd = umma_desc(src + 2 * kh * kSPlane + dx * 16, kSPlane, 128);
-                        asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(dst + (uint32_t)(dx * 16 + kh * 8)),
-                                     "l"(sd)
-                                     : "memory");
-                    }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&rcp[sl]))
-                             : "memory");
-                s_copies = qq + 1;
-                return true;
-            };
-            auto copied = [&](int qq) {
-                return mbar_wait(smem_u32(&rcp[qq % kSRows]), (uint32_t)((qq / kSRows) & 1));
-            };
-            for (int i = 0; i < cnt && !s_stop; i++) {
-                int b, sx, y0, y1;
-                strip_item(g, (int)blockIdx.x + i * (int)gridDim.x, b, sx, y0, y1);
-                (void)b;
-                (void)sx;
-                const int q0 = q;                      // sequence number of input row y0 - 1
-                // the previous item's MMAs are complete before its TMEM rows are overwritten
-                if (j > 0 && !mbar_wait(smem_u32(&dfull[(j - 1) & 1]), (uint32_t)(((j - 1) >> 1) & 1))) {
-                    s_stop = 1;
-                    break;
-                }
-                bool ok = copy_row(q0) && copy_row(q0 + 1) && copy_row(q0 + 2);
-                q = q0 + 3;
-                for (int y = y0; ok && y < y1; y++, j++) {
-                    const int a = j & 1, r = y - y0;
-                    // the epilogue has read accumulator a (output row j - 2)
-                    if (j >= 2 && !mbar_wait(smem_u32(&dempty[a]), (uint32_t)(((j >> 1) - 1) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    if (!(copied(q0 + r) && copied(q0 + r + 1) && copied(q0 + r + 2))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                    for (int tap = 0; tap < 9; tap++) {
-                        const int dy = tap / 3, dx = tap % 3;
-                        const uint32_t arow = tmem + (uint32_t)(((q0 + r + dy) % kSSlots) * kSSlotCols + dx * 16);
-#pragma unroll
-                        for (int kh = 0; kh < 2; kh++) {
-                            const uint64_t db = umma_desc(wbase + (4 * tap + 2 * kh) * 128, 128, kWRowGroup);
-                            const uint32_t accum = (tap | kh) ? 1u : 0u;
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\t"
-                                "setp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                                ::"r"(tmem + (uint32_t)(kSDcol + a * 32)), "r"(arow + (uint32_t)(kh * 8)), "l"(db),
-                                  "r"(kIdesc), "r"(accum)
-                                : "memory");
-                        }
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(&dfull[a]))
-                                 : "memory");
-                    s_mmas = j + 1;
-                    // input row y + 2 goes into the slot of input row y - 2, which
-                    // output row j - 1 reads last: wait for that row's MMAs (row j's
-                    // are queued behind them), then copy
-                    if (y + 2 <= y1) {
-                        if (j >= 1 && !mbar_wait(smem_u32(&dfull[(j - 1) & 1]), (uint32_t)(((j - 1) >> 1) & 1))) {
-                            ok = false;
-                            break;
-                        }
-                        if (!copy_row(q0 + r + 3)) {
-                            ok = false;
-                            break;
-                        }
-                        q = q0 + r + 4;
-                    }
-                }
-                if (!ok) {
-                    s_stop = 1;
-                    break;
-                }
-            }
-        }
-    } else {
-        const int lg = warp & 3;                       // TMEM lane group of this warp
-        int j = 0;
-        bool ok = true;
-        for (int i = 0; ok && i < cnt; i++) {
-            int b, sx, y0, y1;
-            strip_item(g, (int)blockIdx.x + i * (int)gridDim.x, b, sx, y0, y1);
-            for (int y = y0; y < y1; y++, j++) {
-                const int a = j & 1;
-                ok = !s_stop && mbar_wait(smem_u32(&dfull[a]), (uint32_t)((j >> 1) & 1));
-                if (!__all_sync(0xffffffffu, ok)) {
-                    if (lane == 0) s_stop = 1;
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t r[32];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                    "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                      "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                      "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                      "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                    : "r"(tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)(kSDcol + a * 32))
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&dempty[a]));
-                const int x = sx * kSW + lg * 32 + lane;
-                if (x < g.W) {
-                    const size_t pix = ((size_t)b * g.H + y) * g.W + x;
-                    if constexpr (MODE == kFwdProj)
-                        proj_store(r, pix, (size_t)g.B * g.H * g.W, static_cast<const bf16*>(aux), w6s,
-                                   static_cast<float*>(out));
-                    else
-                        conv_store<MODE>(r, pix * 32, aux, out, out16);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (s_stop && tid == 32) {
-        // report, then let the loads, copies and MMAs still in flight finish (bounded) before TMEM is freed
-        atomicOr(err, 1);
-        const int nl = s_loads, nc = s_copies, nm = s_mmas;
-        for (int k = nc; k < nl; k++) mbar_wait(smem_u32(&rfull[k % kSRows]), (uint32_t)((k / kSRows) & 1));
-        if (nc > 0) mbar_wait(smem_u32(&rcp[(nc - 1) % kSRows]), (uint32_t)(((nc - 1) / kSRows) & 1));
-        if (nm > 0) mbar_wait(smem_u32(&dfull[(nm - 1) & 1]), (uint32_t)(((nm - 1) >> 1) & 1));
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kSTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -1063,136 +781,55 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-// box_c: channels per box (32: the whole 64-byte pixel; 8: one plane)
-static CUtensorMap conv_input_map(int B, int H, int W, const __nv_bfloat16* in, int box_c)
-{
-    CUtensorMap map;
-    const cuuint64_t dims[4] = {32, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {64, (cuuint64_t)W * 64, (cuuint64_t)W * H * 64};
-    const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)kHW, (cuuint32_t)kHH, 1};
-    const cuuint32_t estride[4] = {1, 1, 1, 1};
-    CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(in), dims,
-                                      strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    JFG_CHECK(r == CUDA_SUCCESS, JFG_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-    return map;
-}
-
-// One input row of a strip: box of 8 channels x 130 pixels x 1 row (zero fill
-// outside the image: the x halo at the image edges and rows -1 and H).
-static CUtensorMap conv_row_map(int B, int H, int W, const __nv_bfloat16* in)
-{
-    CUtensorMap map;
-    const cuuint64_t dims[4] = {32, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {64, (cuuint64_t)W * 64, (cuuint64_t)W * H * 64};
-    const cuuint32_t box[4] = {8, (cuuint32_t)kSPx, 1, 1};
-    const cuuint32_t estride[4] = {1, 1, 1, 1};
-    CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(in), dims,
-                                      strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    JFG_CHECK(r == CUDA_SUCCESS, JFG_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-    return map;
-}
-
-// JFEM_CNN_STRIP=1 selects the strip kernel (k_conv_strip, activations in
-// TMEM) for the 32 -> 32 layers
-static bool use_strip()
-{
-    const char* e = getenv("JFEM_CNN_STRIP");
-    return e && e[0] == '1';
-}
-
-// Strip geometry: strips of 128 pixels, segments of rows sized so that the
-// items fill the SMs (one CTA per SM) in whole rounds: at most two items per
-// CTA when the image allows.
-static StripGeo strip_geo(int B, int H, int W)
-{
-    StripGeo g;
-    g.B = B;
-    g.H = H;
-    g.W = W;
-    g.nstrips = (W + kSW - 1) / kSW;
-    const int slots = 2 * sm_count();
-    int nsegs = std::max(1, slots / std::max(1, B * g.nstrips));
-    nsegs = std::min(nsegs, H);
-    g.rs = (H + nsegs - 1) / nsegs;
-    g.nsegs = (H + g.rs - 1) / g.rs;
-    return g;
-}
-
-template <int MODE>
-static void launch_strip(cudaStream_t st, int B, int H, int W, const bf16* in, const bf16* w, const void* aux,
-                         void* out, bf16* out16, int* err, const float* proj = nullptr)
-{
-    JFG_CHECK(((uintptr_t)in & 15) == 0, JFG_ERR_BAD_ARG, "convolution input not 16-byte aligned");
-    const StripGeo g = strip_geo(B, H, W);
-    const long long items = (long long)B * g.nstrips * g.nsegs;
-    JFG_CHECK(items < (1LL << 31), JFG_ERR_UNSUPPORTED, "image too large for the strip convolution");
-    const int grid = (int)std::min<long long>(items, (long long)kSCtasPerSm * sm_count());
-    if (grid <= 0) return;
-    static bool attr = false;
-    if (!attr) {
-        JFG_CUDA(cudaFuncSetAttribute(k_conv_strip<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStripSmem));
-        attr = true;
-    }
-    const CUtensorMap map = conv_row_map(B, H, W, in);
-    k_conv_strip<MODE><<<grid, kSThreads, kStripSmem, st>>>(map, g, w, aux, out, out16, err, proj);
-    JFG_CUDA(cudaGetLastError());
-    note_launch();
-}
-
 // JFEM_CNN_WS=0 selects the single-role kernel (k_conv_mid_tc) instead of the
-// warp-specialised pipeline (k_conv_ws); JFEM_CNN_WS_STAGES = 2, 3 or 4 sets
-// its stages (default kWsDefaultStages)
-constexpr int kWsDefaultStages = 2;
+// warp-specialised pipeline (k_conv_ws)
 static bool use_ws()
 {
     const char* e = getenv("JFEM_CNN_WS");
     return !(e && e[0] == '0');
 }
-static int ws_stages()
-{
-    const char* e = getenv("JFEM_CNN_WS_STAGES");
-    const int v = e ? atoi(e) : kWsDefaultStages;
-    return (v == 2 || v == 3 || v == 4) ? v : kWsDefaultStages;
-}
-static int ws_ctas(int st) { return st == 2 ? ws_ctas_per_sm<2>() : (st == 3 ? ws_ctas_per_sm<3>() : ws_ctas_per_sm<4>()); }
 
-static int conv_grid(int B, int H, int W, const void* in)
+// The input image as TMA boxes: whole pixels of kRX x kBoxRows with the
+// 64-byte swizzle (k_conv_ws), or planes of 8 channels of the 18 x 10 halo
+// (k_conv_mid_tc); zero fill outside the image.
+static CUtensorMap conv_input_map(int B, int H, int W, const __nv_bfloat16* in, bool ws)
 {
-    const long long ntiles = (long long)((W + kTW - 1) / kTW) * ((H + kTH - 1) / kTH) * B;
-    JFG_CHECK(ntiles < (1LL << 31), JFG_ERR_UNSUPPORTED, "image too large for the tensor-core convolution");
-    JFG_CHECK(((uintptr_t)in & 15) == 0, JFG_ERR_BAD_ARG, "convolution input not 16-byte aligned");
-    const int per_sm = use_ws() ? ws_ctas(ws_stages()) : kTcCtasPerSm;
-    return (int)std::min<long long>(ntiles, (long long)sm_count() * per_sm);
-}
-
-template <int MODE, int ST>
-static void launch_ws(cudaStream_t st, int grid, const CUtensorMap& map, int B, int H, int W, const bf16* w,
-                      const void* aux, void* out, bf16* out16, int* err, const float* proj = nullptr)
-{
-    static bool attr = false;
-    if (!attr) {
-        JFG_CUDA(cudaFuncSetAttribute(k_conv_ws<MODE, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws_smem<ST>()));
-        attr = true;
-    }
-    k_conv_ws<MODE, ST><<<grid, kWsThreads, ws_smem<ST>(), st>>>(map, B, H, W, w, aux, out, out16, err, proj);
+    CUtensorMap map;
+    const cuuint64_t dims[4] = {32, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {64, (cuuint64_t)W * 64, (cuuint64_t)W * H * 64};
+    const cuuint32_t box[4] = {ws ? 32u : 8u, (cuuint32_t)(ws ? kRX : kHW), (cuuint32_t)(ws ? kBoxRows : kHH), 1};
+    const cuuint32_t estride[4] = {1, 1, 1, 1};
+    CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(in), dims,
+                                      strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      ws ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    JFG_CHECK(r == CUDA_SUCCESS, JFG_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    return map;
 }
 
 template <int MODE>
-static void launch_conv(cudaStream_t st, int grid, const CUtensorMap& map, int B, int H, int W, const bf16* w,
-                        const void* aux, void* out, bf16* out16, int* err)
+static void launch_conv(cudaStream_t st, int B, int H, int W, const bf16* in, const bf16* w, const void* aux, void* out,
+                        bf16* out16, int* err, const float* proj = nullptr)
 {
-    if (use_ws()) {
-        switch (ws_stages()) {
-        case 2: launch_ws<MODE, 2>(st, grid, map, B, H, W, w, aux, out, out16, err); break;
-        case 3: launch_ws<MODE, 3>(st, grid, map, B, H, W, w, aux, out, out16, err); break;
-        default: launch_ws<MODE, 4>(st, grid, map, B, H, W, w, aux, out, out16, err); break;
+    const bool ws = use_ws();
+    const long long ntiles = ws ? (long long)((W + kOutX - 1) / kOutX) * ((H + kRY - 1) / kRY) * B
+                                : (long long)((W + kTW - 1) / kTW) * ((H + kTH - 1) / kTH) * B;
+    JFG_CHECK(ntiles < (1LL << 30), JFG_ERR_UNSUPPORTED, "image too large for the tensor-core convolution");
+    JFG_CHECK(((uintptr_t)in & 15) == 0, JFG_ERR_BAD_ARG, "convolution input not 16-byte aligned");
+    const int grid = (int)std::min<long long>(ntiles, (long long)sm_count() * (ws ? kDxCtasPerSm : kTcCtasPerSm));
+    if (grid <= 0) return;
+    const CUtensorMap map = conv_input_map(B, H, W, in, ws);
+    if (ws) {
+        static bool attr = false;
+        if (!attr) {
+            JFG_CUDA(cudaFuncSetAttribute(k_conv_ws<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem));
+            attr = true;
         }
-    } else {
+        k_conv_ws<MODE><<<grid, kDxThreads, kDxSmem, st>>>(map, B, H, W, w, aux, out, out16, err, proj);
+    } else if constexpr (MODE != kFwdProj) {
         k_conv_mid_tc<MODE><<<grid, kTcThreads, 0, st>>>(map, B, H, W, w, aux, out, out16, err);
+    } else {
+        JFG_CHECK(false, JFG_ERR_UNSUPPORTED, "the fused output projection needs the warp-specialised convolution");
     }
     JFG_CUDA(cudaGetLastError());
     note_launch();
@@ -1204,20 +841,10 @@ static void launch_conv(cudaStream_t st, int grid, const CUtensorMap& map, int B
 void conv_mid_tc(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* in, const __nv_bfloat16* wk,
                  const __nv_bfloat16* skip, __nv_bfloat16* out, int* err)
 {
-    if (use_strip()) {
-        if (skip)
-            launch_strip<kFwdSkip>(st, B, H, W, in, wk, skip, out, nullptr, err);
-        else
-            launch_strip<kFwd>(st, B, H, W, in, wk, nullptr, out, nullptr, err);
-        return;
-    }
-    const int grid = conv_grid(B, H, W, in);
-    if (grid <= 0) return;
-    const CUtensorMap map = conv_input_map(B, H, W, in, use_ws() ? 32 : 8);
     if (skip)
-        launch_conv<kFwdSkip>(st, grid, map, B, H, W, wk, skip, out, nullptr, err);
+        launch_conv<kFwdSkip>(st, B, H, W, in, wk, skip, out, nullptr, err);
     else
-        launch_conv<kFwd>(st, grid, map, B, H, W, wk, nullptr, out, nullptr, err);
+        launch_conv<kFwd>(st, B, H, W, in, wk, nullptr, out, nullptr, err);
 }
 
 // The last 32 -> 32 layer with its skip input fused with the projection of
@@ -1225,26 +852,12 @@ void conv_mid_tc(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* in, 
 // entries, u[t][p] = sum_c w6[c][t] relu(conv + skip)[p][c] (BF16-rounded
 // activations); w6 is FP32 [32 channels][9 taps].  Warp-specialised kernel
 // only (the caller checks conv_proj_available()).
-bool conv_proj_available() { return use_strip() || use_ws(); }
+bool conv_proj_available() { return use_ws(); }
 
 void conv_mid_tc_proj(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* in, const __nv_bfloat16* wk,
                       const __nv_bfloat16* skip, const float* w6, float* u, int* err)
 {
-    if (use_strip()) {
-        launch_strip<kFwdProj>(st, B, H, W, in, wk, skip, u, nullptr, err, w6);
-        return;
-    }
-    const int grid = conv_grid(B, H, W, in);
-    if (grid <= 0) return;
-    JFG_CHECK(use_ws(), JFG_ERR_UNSUPPORTED, "the fused output projection needs the warp-specialised convolution");
-    const CUtensorMap map = conv_input_map(B, H, W, in, 32);
-    switch (ws_stages()) {
-    case 2: launch_ws<kFwdProj, 2>(st, grid, map, B, H, W, wk, skip, u, nullptr, err, w6); break;
-    case 3: launch_ws<kFwdProj, 3>(st, grid, map, B, H, W, wk, skip, u, nullptr, err, w6); break;
-    default: launch_ws<kFwdProj, 4>(st, grid, map, B, H, W, wk, skip, u, nullptr, err, w6); break;
-    }
-    JFG_CUDA(cudaGetLastError());
-    note_launch();
+    launch_conv<kFwdProj>(st, B, H, W, in, wk, skip, u, nullptr, err, w6);
 }
 
 // Input gradient of a 32 -> 32 layer on the tensor cores: conv3x3 of the
@@ -1254,20 +867,10 @@ void conv_mid_tc_proj(cudaStream_t st, int B, int H, int W, const __nv_bfloat16*
 void conv_mid_tc_bwd(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* gin, const __nv_bfloat16* wt,
                      const __nv_bfloat16* mask, const float* skip, float* out, __nv_bfloat16* out16, int* err)
 {
-    if (use_strip()) {
-        if (mask)
-            launch_strip<kBwdMask>(st, B, H, W, gin, wt, mask, out, out16, err);
-        else
-            launch_strip<kBwdSkip>(st, B, H, W, gin, wt, skip, out, nullptr, err);
-        return;
-    }
-    const int grid = conv_grid(B, H, W, gin);
-    if (grid <= 0) return;
-    const CUtensorMap map = conv_input_map(B, H, W, gin, use_ws() ? 32 : 8);
     if (mask)
-        launch_conv<kBwdMask>(st, grid, map, B, H, W, wt, mask, out, out16, err);
+        launch_conv<kBwdMask>(st, B, H, W, gin, wt, mask, out, out16, err);
     else
-        launch_conv<kBwdSkip>(st, grid, map, B, H, W, wt, skip, out, nullptr, err);
+        launch_conv<kBwdSkip>(st, B, H, W, gin, wt, skip, out, nullptr, err);
 }
 
 // Per-CTA partial weight gradients of a 32 -> 32 layer on the tensor cores

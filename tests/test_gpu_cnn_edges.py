@@ -30,3 +30,24 @@ def test_edge_layer_weight_gradients(ctx, shape):
     for l in (0, 5):
         err = np.linalg.norm(gg[l] - gr[l]) / np.linalg.norm(gr[l])
         assert err < TOL, (l, err)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 3, 29), (1, 4, 30), (1, 5, 31), (3, 8, 60), (1, 9, 61), (1, 70, 91)])
+def test_conv_tiles_of_four_rows_of_thirty(ctx, shape, monkeypatch):
+    """k_conv_ws tiles (4 rows x 30 output pixels) at their edges: forward and
+    gradients equal the single-role kernel's bit for bit (16 x 8 tiles, the
+    same accumulators), and the forward the rounding oracle."""
+    rng = np.random.default_rng(32)
+    w = he_init(seed=12, gain_last=1.0)
+    xh = rng.standard_normal(shape).astype(np.float32)
+    x = torch.from_numpy(xh).cuda()
+    t = torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda()
+    net = LearnedSmoother(ctx, w)
+    monkeypatch.setenv("JFEM_CNN_PROJ", "0")
+    outs = []
+    for ws in ("1", "0"):
+        monkeypatch.setenv("JFEM_CNN_WS", ws)
+        outs.append((net.forward(x).cpu().numpy(), net.loss_and_grad(x, t)[1]))
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+    yr, _ = CO.forward_bf16(unpack(w), xh.astype(np.float64))
+    assert np.linalg.norm(outs[0][0] - yr) < TOL * np.linalg.norm(yr)
