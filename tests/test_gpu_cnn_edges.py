@@ -51,3 +51,23 @@ def test_conv_tiles_of_four_rows_of_thirty(ctx, shape, monkeypatch):
     assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
     yr, _ = CO.forward_bf16(unpack(w), xh.astype(np.float64))
     assert np.linalg.norm(outs[0][0] - yr) < TOL * np.linalg.norm(yr)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 7, 15), (1, 8, 16), (1, 9, 17), (3, 17, 33), (2, 200, 130)])
+def test_tensor_core_weight_gradients_at_tile_edges(ctx, shape, monkeypatch):
+    """k_wgrad_tc tiles (8 rows x 16 pixels, G with a halo row each side) at
+    their edges and with several tiles per CTA, against the mma.sync kernel on
+    the same BF16 images: FP32 sums of the same products in another order."""
+    rng = np.random.default_rng(33)
+    w = he_init(seed=13, gain_last=1.0)
+    x = torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda()
+    net = LearnedSmoother(ctx, w)
+    g = []
+    for tc in ("1", "0"):
+        monkeypatch.setenv("JFEM_CNN_WGRAD_TC", tc)
+        g.append(unpack(net.loss_and_grad(x, t)[1]))
+    for l in (1, 2, 3, 4):
+        # n products per entry: random-walk growth of the FP32 rounding of their sums
+        bound = 2.0 ** -23 * np.sqrt(np.prod(shape) + 16.0) * 4
+        assert np.linalg.norm(g[0][l] - g[1][l]) <= bound * np.linalg.norm(g[1][l]) + 1e-30, l
