@@ -451,31 +451,68 @@ struct FinLoss {
     __device__ void operator()(const double* s) const { *out = s[0] * invn; }
 };
 
-// dh5[p][ci] = sum_tap w6[ci][tap] dy[p - (tap - 4 offset)]  (input gradient of conv6)
-__global__ void k_conv_out_bwd(int B, int H, int W, const float* __restrict__ dy, const float* __restrict__ w6,
-                               float* __restrict__ dh5)
+// g5 = dh5 * (h5 > 0) with dh5[p][ci] = sum_tap w6[ci][tap] dy[p - tap] (the
+// input gradient of conv6 through the ReLU before it), in FP32 and, where g16
+// is given, its BF16 copy.  The scheme of k_conv_in: four lanes per pixel,
+// eight channels each with their 72 weights in registers, a 3 x 3 window that
+// slides down kInRows rows (the window runs against the taps).  One thread per
+// pixel, its 32 channels stored one by one, took 45 us and the mask in a
+// kernel of its own 31 us more at 16 x 128 x 128 pixels.
+__global__ void __launch_bounds__(256)
+k_conv_out_bwd(int B, int H, int W, const float* __restrict__ dy, const float* __restrict__ w6,
+               const bf16* __restrict__ h5, float* __restrict__ g, bf16* __restrict__ g16)
 {
-    __shared__ float ws[kC * 9];
-    for (int i = threadIdx.x; i < kC * 9; i += blockDim.x) ws[i] = w6[i];
+    __shared__ __align__(16) float ws[9 * kC];
+    for (int i = threadIdx.x; i < kC * 9; i += blockDim.x) ws[(i % 9) * kC + i / 9] = w6[i];
     __syncthreads();
-    const size_t npx = (size_t)B * H * W;
-    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += (size_t)gridDim.x * blockDim.x) {
-        const int xx = (int)(p % W), yy = (int)((p / W) % H);
-        const size_t bb = p / ((size_t)H * W);
-        float g9[9];
+    const int xx = blockIdx.x * kEdgePx + (int)threadIdx.x / kLanesPerPx, q = threadIdx.x % kLanesPerPx;
+    const int ry = (H + kInRows - 1) / kInRows;
+    const int bb = blockIdx.y / ry, y0 = (blockIdx.y - bb * ry) * kInRows;
+    if (xx >= W) return;
+    float w[9][8];
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) w[tap][c] = ws[tap * kC + 8 * q + c];
+    const float* db = dy + (size_t)bb * H * W;
+    auto row3 = [&](int yy, float (&v)[3]) {
+        const bool okr = yy >= 0 && yy < H;
+#pragma unroll
+        for (int dx = -1; dx <= 1; dx++)
+            v[dx + 1] = okr && xx + dx >= 0 && xx + dx < W ? __ldg(db + (size_t)yy * W + xx + dx) : 0.f;
+    };
+    float win[3][3];
+    row3(y0 - 1, win[0]);
+    row3(y0, win[1]);
+    const int y1 = min(H, y0 + kInRows);
+    for (int yy = y0; yy < y1; yy++) {
+        row3(yy + 1, win[2]);
+        const size_t base = (((size_t)bb * H + yy) * W + xx) * kC + 8 * q;
+        const uint4 hm = __ldg(reinterpret_cast<const uint4*>(h5 + base));
+        const uint32_t hw[4] = {hm.x, hm.y, hm.z, hm.w};
+        float s[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) s[c] = 0.f;
 #pragma unroll
         for (int tap = 0; tap < 9; tap++) {
-            // dx[q] += w[tap] g[q - (dy-1, dx-1)]
-            int gy = yy - (tap / 3 - 1), gx = xx - (tap % 3 - 1);
-            g9[tap] = (gy >= 0 && gy < H && gx >= 0 && gx < W) ? dy[(bb * H + gy) * W + gx] : 0.f;
-        }
-        float* o = dh5 + p * kC;
-#pragma unroll 4
-        for (int ci = 0; ci < kC; ci++) {
-            float s = 0.f;
+            const float in = win[2 - tap / 3][2 - tap % 3];
 #pragma unroll
-            for (int tap = 0; tap < 9; tap++) s += ws[ci * 9 + tap] * g9[tap];
-            o[ci] = s;
+            for (int c = 0; c < 8; c++) s[c] += w[tap][c] * in;
+        }
+        __align__(16) bf16 o[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const uint32_t u = hw[c >> 1];
+            if (!(__uint_as_float(c & 1 ? u & 0xFFFF0000u : u << 16) > 0.f)) s[c] = 0.f;
+            o[c] = __float2bfloat16_rn(s[c]);
+        }
+        *reinterpret_cast<float4*>(g + base) = make_float4(s[0], s[1], s[2], s[3]);
+        *reinterpret_cast<float4*>(g + base + 4) = make_float4(s[4], s[5], s[6], s[7]);
+        if (g16) *reinterpret_cast<uint4*>(g16 + base) = *reinterpret_cast<const uint4*>(o);
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            win[0][e] = win[1][e];
+            win[1][e] = win[2][e];
         }
     }
 }
@@ -590,16 +627,12 @@ __global__ void __launch_bounds__(1024) k_wgrad_edge_reduce(int nparts, const fl
     if (threadIdx.x < 32) dw[i] = s;
 }
 
-// g = d * (a > 0), and g16 = the same in BF16 when given (the TMA input of
-// the tensor-core input-gradient convolution)
-__global__ void k_relu_mask(size_t n, const float* __restrict__ d, const bf16* __restrict__ a, float* __restrict__ g,
-                            bf16* __restrict__ g16)
+// g = d * (a > 0): the ReLU mask after an mma.sync input gradient with skip
+// (the tensor-core kernels apply it in their epilogue)
+__global__ void k_relu_mask(size_t n, const float* __restrict__ d, const bf16* __restrict__ a, float* __restrict__ g)
 {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = __bfloat162float(a[i]) > 0.f ? d[i] : 0.f;
-        g[i] = v;
-        if (g16) g16[i] = __float2bfloat16_rn(v);
-    }
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        g[i] = __bfloat162float(a[i]) > 0.f ? d[i] : 0.f;
 }
 
 // BF16 weight layouts from the FP32 master (co, ci, dy, dx):
@@ -819,45 +852,42 @@ void cnn_backward(jfg_cnn* n, cudaStream_t st, int B, int H, int W, const float*
     const int ectas = edge_ctas(B, H, W);
     k_wgrad_edge<1><<<ectas, 256, 0, st>>>(B, H, W, nullptr, n->dy.p, n->h5.p, n->part.p);
     k_wgrad_edge_reduce<<<9, 1024, 0, st>>>(ectas, n->part.p, g + kLayerOff[5]);
-    k_conv_out_bwd<<<grid1d(npx), 256, 0, st>>>(B, H, W, n->dy.p, n->w32.p + kLayerOff[5], n->gA.p);
     // input gradients on the tensor cores (BF16 copies of the gradient images
     // as their TMA inputs) unless JFEM_CNN_TC=0 selects the mma.sync kernels;
-    // both round the gradient images to BF16 for the products
+    // both round the gradient images to BF16 for the products.  An FP32 image
+    // that only the mma.sync weight gradient would read (g4, g2) is not written
+    // where the tensor-core one runs.
     const bool tc = use_tc();
     bf16* gB16 = tc ? n->gB16.p : nullptr;
+    float* gC = tc && wgrad_tc_enabled() ? nullptr : n->gC.p;
     int* err = n->tc_err.p;
-    k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h5.p, n->gB.p, gB16);      // g5
+    const dim3 out_grid((unsigned)((W + kEdgePx - 1) / kEdgePx), (unsigned)(B * ((H + kInRows - 1) / kInRows)));
+    k_conv_out_bwd<<<out_grid, 256, 0, st>>>(B, H, W, n->dy.p, n->w32.p + kLayerOff[5], n->h5.p, n->gB.p, gB16);   // g5
     JFG_CUDA(cudaGetLastError());
     wgrad_mid(n, st, B, H, W, n->gB.p, gB16, n->a4.p, g + kLayerOff[4]);                            // dW5
-    if (tc)
-        conv_mid_tc_bwd(st, B, H, W, gB16, wt + 3 * kMidParams, n->a4.p, nullptr, n->gC.p, n->gC16.p, err);
-    else
-        conv_mid<float, float, 0, false, true>(st, B, H, W, n->gB.p, wt + 3 * kMidParams, nullptr, n->a4.p,
-                                               n->gC.p);                                            // g4
-    wgrad_mid(n, st, B, H, W, n->gC.p, tc ? n->gC16.p : nullptr, n->h3.p, g + kLayerOff[3]);     // dW4
-    if (tc)
-        conv_mid_tc_bwd(st, B, H, W, n->gC16.p, wt + 2 * kMidParams, nullptr, n->gB.p, n->gA.p, nullptr, err);
-    else
-        conv_mid<float, float, 2, false, false>(st, B, H, W, n->gC.p, wt + 2 * kMidParams, n->gB.p, nullptr,
-                                                n->gA.p);                                           // dh3
-    k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h3.p, n->gB.p, gB16);      // g3
-    wgrad_mid(n, st, B, H, W, n->gB.p, gB16, n->a2.p, g + kLayerOff[2]);                            // dW3
-    if (tc)
-        conv_mid_tc_bwd(st, B, H, W, gB16, wt + 1 * kMidParams, n->a2.p, nullptr, n->gC.p, n->gC16.p, err);
-    else
-        conv_mid<float, float, 0, false, true>(st, B, H, W, n->gB.p, wt + 1 * kMidParams, nullptr, n->a2.p,
-                                               n->gC.p);                                            // g2
-    wgrad_mid(n, st, B, H, W, n->gC.p, tc ? n->gC16.p : nullptr, n->h1.p, g + kLayerOff[1]);     // dW2
-    if (tc)
-        conv_mid_tc_bwd(st, B, H, W, n->gC16.p, wt + 0 * kMidParams, nullptr, n->gB.p, n->gA.p, nullptr, err);
-    else
-        conv_mid<float, float, 2, false, false>(st, B, H, W, n->gC.p, wt + 0 * kMidParams, n->gB.p, nullptr,
-                                                n->gA.p);                                           // dh1
-    k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h1.p, n->gB.p, nullptr);   // g1
+    if (tc) {
+        conv_mid_tc_bwd(st, B, H, W, gB16, wt + 3 * kMidParams, n->a4.p, nullptr, gC, n->gC16.p, err);       // g4
+        wgrad_mid(n, st, B, H, W, gC, n->gC16.p, n->h3.p, g + kLayerOff[3]);                        // dW4
+        conv_mid_tc_bwd(st, B, H, W, n->gC16.p, wt + 2 * kMidParams, n->h3.p, n->gB.p, n->gA.p, gB16, err);  // g3
+        wgrad_mid(n, st, B, H, W, n->gA.p, gB16, n->a2.p, g + kLayerOff[2]);                        // dW3
+        conv_mid_tc_bwd(st, B, H, W, gB16, wt + 1 * kMidParams, n->a2.p, nullptr, gC, n->gC16.p, err);       // g2
+        wgrad_mid(n, st, B, H, W, gC, n->gC16.p, n->h1.p, g + kLayerOff[1]);                        // dW2
+        conv_mid_tc_bwd(st, B, H, W, n->gC16.p, wt + 0 * kMidParams, n->h1.p, n->gA.p, n->gB.p, nullptr, err);  // g1
+    } else {
+        conv_mid<float, float, 0, false, true>(st, B, H, W, n->gB.p, wt + 3 * kMidParams, nullptr, n->a4.p, gC);
+        wgrad_mid(n, st, B, H, W, gC, nullptr, n->h3.p, g + kLayerOff[3]);                          // dW4
+        conv_mid<float, float, 2, false, false>(st, B, H, W, gC, wt + 2 * kMidParams, n->gB.p, nullptr, n->gA.p);
+        k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h3.p, n->gB.p);         // g3
+        wgrad_mid(n, st, B, H, W, n->gB.p, nullptr, n->a2.p, g + kLayerOff[2]);                     // dW3
+        conv_mid<float, float, 0, false, true>(st, B, H, W, n->gB.p, wt + 1 * kMidParams, nullptr, n->a2.p, gC);
+        wgrad_mid(n, st, B, H, W, gC, nullptr, n->h1.p, g + kLayerOff[1]);                          // dW2
+        conv_mid<float, float, 2, false, false>(st, B, H, W, gC, wt + 0 * kMidParams, n->gB.p, nullptr, n->gA.p);
+        k_relu_mask<<<grid1d(npx * kC), 256, 0, st>>>(npx * kC, n->gA.p, n->h1.p, n->gB.p);         // g1
+    }
     k_wgrad_edge<0><<<ectas, 256, 0, st>>>(B, H, W, n->gB.p, x, nullptr, n->part.p);
     k_wgrad_edge_reduce<<<9, 1024, 0, st>>>(ectas, n->part.p, g + kLayerOff[0]);
     JFG_CUDA(cudaGetLastError());
-    note_launch(9);
+    note_launch(tc ? 5 : 7);
 }
 
 }  // namespace

@@ -92,7 +92,10 @@ __device__ __forceinline__ void tma_plane(uint32_t dst, const CUtensorMap* map, 
 //   kBwdMask: out(f32) = acc * (mask(bf16) > 0), out16 = the same in BF16
 //             (an input gradient through the next layer's ReLU, and its BF16
 //             copy: the TMA input of the following input-gradient convolution)
-//   kBwdSkip: out(f32) = acc + skip(f32)                     input gradient plus the skip path's
+//             (out may be null: only the BF16 image is wanted)
+//   kBwdSkip: g = (acc + skip(f32)) * (mask(bf16) > 0): the input gradient plus
+//             the skip path's through the ReLU of the layer before; out(f32) = g
+//             and, where out16 is given, its BF16 copy
 //   kFwdProj: the last 32 -> 32 layer (with skip) fused with the projection of
 //   the 32 -> 1 output layer: h = relu(acc + skip) rounded to BF16 (the values
 //   the output layer would read back), then u[t][p] = sum_c w6[c][t] h[c] for
@@ -101,13 +104,25 @@ __device__ __forceinline__ void tma_plane(uint32_t dst, const CUtensorMap* map, 
 constexpr int kFwd = 0, kFwdSkip = 1, kBwdMask = 2, kBwdSkip = 3, kFwdProj = 4;
 
 // The image a mode's epilogue reads beside the accumulator, one pixel: 32
-// BF16 (skip or mask) or 32 FP32 (skip) channels.
+// BF16 (skip or mask) or 32 FP32 (skip; the mask beside it) channels.
 template <int MODE>
 struct AuxPx {
     static constexpr int kVecs = MODE == kFwd ? 0 : (MODE == kBwdSkip ? 8 : 4);
     uint4 q[kVecs ? kVecs : 1];
-    __device__ __forceinline__ void load(const void* __restrict__ aux, size_t pix, bool inside)
+    uint4 m[MODE == kBwdSkip ? 4 : 1];
+    __device__ __forceinline__ bool keep(int c) const     // kBwdSkip: the mask of channel c
     {
+        const uint32_t u = reinterpret_cast<const uint32_t*>(m)[c >> 1];
+        return __uint_as_float(c & 1 ? u & 0xFFFF0000u : u << 16) > 0.f;
+    }
+    __device__ __forceinline__ void load(const void* __restrict__ aux, const bf16* __restrict__ mask, size_t pix,
+                                         bool inside)
+    {
+        if constexpr (MODE == kBwdSkip) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                m[i] = inside ? __ldg(reinterpret_cast<const uint4*>(mask) + pix * 4 + i) : make_uint4(0, 0, 0, 0);
+        }
 #pragma unroll
         for (int i = 0; i < kVecs; i++)
             q[i] = inside ? __ldg(reinterpret_cast<const uint4*>(aux) + pix * kVecs + i) : make_uint4(0, 0, 0, 0);
@@ -146,10 +161,11 @@ __device__ __forceinline__ void conv_emit(const float (&v)[16], int c0, const Au
         if (MODE == kFwd) f[c] = fmaxf(v[c], 0.f);
         if (MODE == kFwdSkip) f[c] = fmaxf(v[c] + aux.at(c0 + c), 0.f);
         if (MODE == kBwdMask) f[c] = aux.at(c0 + c) > 0.f ? v[c] : 0.f;
-        if (MODE == kBwdSkip) f[c] = v[c] + aux.at(c0 + c);
+        if (MODE == kBwdSkip) f[c] = aux.keep(c0 + c) ? v[c] + aux.at(c0 + c) : 0.f;
     }
     const size_t base = pix * 32 + c0;
-    if (MODE == kBwdMask || MODE == kBwdSkip) {
+    constexpr bool bwd = MODE == kBwdMask || MODE == kBwdSkip;
+    if (bwd && out) {
         float* of = static_cast<float*>(out) + base;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -159,11 +175,11 @@ __device__ __forceinline__ void conv_emit(const float (&v)[16], int c0, const Au
             st_sector(of + 8 * h, w);
         }
     }
-    if (MODE != kBwdSkip) {
+    if (!bwd || out16) {
         uint32_t w[8];
 #pragma unroll
         for (int c = 0; c < 8; c++) w[c] = pack_bf16(f[2 * c], f[2 * c + 1]);
-        st_sector((MODE == kBwdMask ? out16 : static_cast<bf16*>(out)) + base, w);
+        st_sector((bwd ? out16 : static_cast<bf16*>(out)) + base, w);
     }
 }
 
@@ -185,7 +201,8 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads)
 k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf16* __restrict__ wk,
-              const void* __restrict__ aux, void* __restrict__ out, bf16* __restrict__ out16, int* __restrict__ err)
+              const void* __restrict__ aux, const bf16* __restrict__ mask, void* __restrict__ out,
+              bf16* __restrict__ out16, int* __restrict__ err)
 {
     __shared__ __align__(128) unsigned char wsm[kWBytes];
     __shared__ __align__(128) unsigned char halo[kStages][kHaloBytes];
@@ -313,7 +330,7 @@ k_conv_mid_tc(const __grid_constant__ CUtensorMap tin, int B, int H, int W, cons
         const bool inside = gy < H && gx < W;
         const size_t pix = inside ? ((size_t)b * H + gy) * W + gx : 0;
         AuxPx<MODE> ax;
-        ax.load(aux, pix, inside);
+        ax.load(aux, mask, pix, inside);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(s * 128 + 16 * h);
@@ -401,8 +418,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 template <int MODE>
 __global__ void __launch_bounds__(kDxThreads, kDxCtasPerSm)
 k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf16* __restrict__ wk,
-          const void* __restrict__ aux, void* __restrict__ out, bf16* __restrict__ out16, int* __restrict__ err,
-          const float* __restrict__ proj)
+          const void* __restrict__ aux, const bf16* __restrict__ mask, void* __restrict__ out,
+          bf16* __restrict__ out16, int* __restrict__ err, const float* __restrict__ proj)
 {
     extern __shared__ unsigned char dsm_raw[];
     unsigned char* boxes = reinterpret_cast<unsigned char*>(((uintptr_t)dsm_raw + 1023) & ~(uintptr_t)1023);
@@ -514,7 +531,7 @@ k_conv_ws(const __grid_constant__ CUtensorMap tin, int B, int H, int W, const bf
             const bool inside = gy < H && gx < W && lane >= 1 && lane <= kOutX;
             const size_t pix = inside ? ((size_t)b * H + gy) * W + gx : 0;
             AuxPx<MODE> ax;
-            ax.load(aux, pix, inside);
+            ax.load(aux, mask, pix, inside);
             const bool ok = !s_stop && mbar_wait(smem_u32(&tfull[a]), (uint32_t)((i / kDxAcc) & 1));
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) s_stop = 1;
@@ -790,7 +807,7 @@ static CUtensorMap conv_input_map(int B, int H, int W, const __nv_bfloat16* in, 
 
 template <int MODE>
 static void launch_conv(cudaStream_t st, int B, int H, int W, const bf16* in, const bf16* w, const void* aux, void* out,
-                        bf16* out16, int* err, const float* proj = nullptr)
+                        bf16* out16, int* err, const float* proj = nullptr, const bf16* mask = nullptr)
 {
     const bool ws = use_ws();
     const long long ntiles = ws ? (long long)((W + kOutX - 1) / kOutX) * ((H + kRY - 1) / kRY) * B
@@ -806,9 +823,9 @@ static void launch_conv(cudaStream_t st, int B, int H, int W, const bf16* in, co
             JFG_CUDA(cudaFuncSetAttribute(k_conv_ws<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem));
             attr = true;
         }
-        k_conv_ws<MODE><<<grid, kDxThreads, kDxSmem, st>>>(map, B, H, W, w, aux, out, out16, err, proj);
+        k_conv_ws<MODE><<<grid, kDxThreads, kDxSmem, st>>>(map, B, H, W, w, aux, mask, out, out16, err, proj);
     } else if constexpr (MODE != kFwdProj) {
-        k_conv_mid_tc<MODE><<<grid, kTcThreads, 0, st>>>(map, B, H, W, w, aux, out, out16, err);
+        k_conv_mid_tc<MODE><<<grid, kTcThreads, 0, st>>>(map, B, H, W, w, aux, mask, out, out16, err);
     } else {
         JFG_CHECK(false, JFG_ERR_UNSUPPORTED, "the fused output projection needs the warp-specialised convolution");
     }
@@ -843,15 +860,15 @@ void conv_mid_tc_proj(cudaStream_t st, int B, int H, int W, const __nv_bfloat16*
 
 // Input gradient of a 32 -> 32 layer on the tensor cores: conv3x3 of the
 // BF16 gradient image gin with the flipped, channel-transposed weights wt
-// (the layout of wk), FP32 accumulation.  mask != nullptr: out = acc *
-// (mask > 0) and out16 = its BF16 copy; else out = acc + skip (FP32).
+// (the layout of wk), FP32 accumulation.  g = (acc [+ skip]) * (mask > 0): out
+// = g in FP32 (null: not wanted), out16 = its BF16 copy (null: not wanted).
 void conv_mid_tc_bwd(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* gin, const __nv_bfloat16* wt,
                      const __nv_bfloat16* mask, const float* skip, float* out, __nv_bfloat16* out16, int* err)
 {
-    if (mask)
-        launch_conv<kBwdMask>(st, B, H, W, gin, wt, mask, out, out16, err);
+    if (skip)
+        launch_conv<kBwdSkip>(st, B, H, W, gin, wt, skip, out, out16, err, nullptr, mask);
     else
-        launch_conv<kBwdSkip>(st, B, H, W, gin, wt, skip, out, nullptr, err);
+        launch_conv<kBwdMask>(st, B, H, W, gin, wt, mask, out, out16, err);
 }
 
 // Per-CTA partial weight gradients of a 32 -> 32 layer on the tensor cores
