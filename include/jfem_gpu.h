@@ -378,13 +378,13 @@ int jfg_solve_dev(jfg_ctx* ctx, int kind, jfg_mat* A, int precond_kind, void* pr
  * reduce across the cluster through distributed shared memory. */
 typedef struct jfg_batch jfg_batch;
 typedef struct {
-    int cluster;        /* CTAs per system (1, 2, 4, 8); 0 = autotuned */
-    int threads;        /* threads per CTA (256, 512); 0 = autotuned */
+    int cluster;        /* CTAs per system (1, 2, 4, 8); 0 = picked by the library */
+    int threads;        /* threads per CTA (256, 512); 0 = picked by the library */
     double rtol;        /* relative FP64 residual per step (default 1e-10) */
     double inner_rtol;  /* FP32 inner PCG relative tolerance (default 1e-5) */
     int inner_max;      /* inner iteration cap (default 500) */
     int max_refine;     /* refinement steps per time step (default 6) */
-    int rows_per_thread; /* rows of a thread in flight per inner pass (2, 3, 4); 0 = autotuned */
+    int rows_per_thread; /* rows of a thread in flight per inner pass (2, 3, 4); 0 = picked by the library */
 } jfg_batch_opts;
 typedef struct {
     int total_inner_iterations;
