@@ -93,3 +93,22 @@ def test_direct_solver_caches_patch_inverses(ctx):
     np.testing.assert_allclose(ds.solve(DenseMatrix(2 * a, ctx), b, 4), np.linalg.solve(2 * a, b), rtol=1e-12,
                                atol=1e-13)
     assert sorted(ds.inverses) == [3, 4]
+
+
+@pytest.mark.parametrize("n", [34, 95, 511, 512, 513, 545, 1025, 1537, 2049])
+def test_blocked_lu_at_panel_edges(ctx, monkeypatch, n):
+    """Panels of one row per thread (512 rows per CTA), ragged last panels and
+    blocks of the cluster solve: the solution equals the column loop's bit for
+    bit; a column of zeros in a later panel is reported as singular."""
+    rng = np.random.default_rng(200 + n)
+    a = rng.standard_normal((n, n))
+    b = rng.standard_normal(n)
+    outs = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("JFEM_LU_BLOCKED", flag)
+        outs.append(DenseMatrix(a, ctx).solve(b))
+    assert np.array_equal(outs[0], outs[1])
+    monkeypatch.setenv("JFEM_LU_BLOCKED", "1")
+    a[:, n - 2] = 0.0
+    with pytest.raises(SingularMatrixException):
+        DenseMatrix(a, ctx).solve(b)
