@@ -361,6 +361,53 @@ constexpr int kBatchRows = 1024;      // patch rows per batch of k_schwarz_batch
 constexpr int kColThreads = 1024;
 constexpr size_t kColSmemMax = 226 * 1024;
 
+// acc[q] = sum_j At(j) * sr[q * m + j] in ascending j for the NP patches of a
+// batch, At(j) = inverse(i, j).  NP is a constant so that the loop has no branch
+// and a chunk's loads are issued before its FP64 chain (~10 cycles per entry):
+// with the number of patches tested inside the loop an entry took ~140 cycles.
+// sr is 16-byte aligned: one patch reads it in pairs (its broadcasts are half of
+// the shared-memory traffic of this loop otherwise).
+template <int NP, class LD>
+__device__ __forceinline__ void inverse_row(int m, const double* sr, LD At, double (&acc)[kMaxBatch])
+{
+#pragma unroll
+    for (int q = 0; q < kMaxBatch; q++) acc[q] = 0.0;
+    int j = 0;
+    if constexpr (NP == 1) {
+#pragma unroll 1
+        for (; j + 8 <= m; j += 8) {
+            double a[8];
+            double2 s[4];
+#pragma unroll
+            for (int u = 0; u < 8; u++) a[u] = At(j + u);
+#pragma unroll
+            for (int u = 0; u < 4; u++) s[u] = *reinterpret_cast<const double2*>(sr + j + 2 * u);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                acc[0] += a[2 * u] * s[u].x;
+                acc[0] += a[2 * u + 1] * s[u].y;
+            }
+        }
+    }
+#pragma unroll (NP == 1 ? 1 : 8)
+    for (; j < m; j++) {
+        const double av = At(j);
+#pragma unroll
+        for (int q = 0; q < NP; q++) acc[q] += av * sr[q * m + j];
+    }
+}
+template <class LD>
+__device__ __forceinline__ void inverse_row(int np, int m, const double* sr, LD At, double (&acc)[kMaxBatch])
+{
+    static_assert(kMaxBatch == 4, "one case per batch size");
+    switch (np) {
+    case 1: inverse_row<1>(m, sr, At, acc); break;
+    case 2: inverse_row<2>(m, sr, At, acc); break;
+    case 3: inverse_row<3>(m, sr, At, acc); break;
+    default: inverse_row<4>(m, sr, At, acc); break;
+    }
+}
+
 template <typename T, typename IT, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT)
     k_schwarz_batch(CsrView A, const int* __restrict__ bpat, const int* __restrict__ bptr,
@@ -370,7 +417,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
 {
     if (done && *done) return;
     __shared__ int sdof[kBatchRows], srs[kBatchRows], sre[kBatchRows];
-    __shared__ double sr[kBatchRows];
+    __shared__ __align__(16) double sr[kBatchRows];
     const int tid = threadIdx.x;
     const int q0 = bptr[blockIdx.x];
     const int np_ = bptr[blockIdx.x + 1] - q0;
@@ -390,15 +437,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     const IT* At = inv + inv_off[p0];                   // transposed: At[j * m + i] = inverse(i, j)
     for (int i = tid; i < m; i += blockDim.x) {
         double acc[kMaxBatch];
-#pragma unroll
-        for (int q = 0; q < kMaxBatch; q++) acc[q] = 0.0;
-#pragma unroll 16
-        for (int j = 0; j < m; j++) {
-            const double a = (double)__ldg(At + (size_t)j * m + i);
-#pragma unroll
-            for (int q = 0; q < kMaxBatch; q++)
-                if (q < np_) acc[q] += a * sr[q * m + j];
-        }
+        inverse_row(np_, m, sr, [&](int j) { return (double)__ldg(At + (size_t)j * m + i); }, acc);
 #pragma unroll
         for (int q = 0; q < kMaxBatch; q++)
             if (q < np_) {
@@ -476,15 +515,8 @@ __global__ void __launch_bounds__(kColThreads, 1)
         const IT* Ag = inv + off;
         for (int i = tid; i < m; i += blockDim.x) {               // sAt[j * m + i] = inverse(i, j)
             double acc[kMaxBatch];
-#pragma unroll
-            for (int q = 0; q < kMaxBatch; q++) acc[q] = 0.0;
-#pragma unroll 16
-            for (int j = 0; j < m; j++) {
-                const double a = SM ? (double)sAt[(size_t)j * m + i] : (double)__ldg(Ag + (size_t)j * m + i);
-#pragma unroll
-                for (int q = 0; q < kMaxBatch; q++)
-                    if (q < np_) acc[q] += a * sr[q * m + j];
-            }
+            inverse_row(np_, m, sr, [&](int j) { return SM ? (double)sAt[j * m + i] : (double)__ldg(Ag + (size_t)j * m + i); },
+                        acc);
 #pragma unroll
             for (int q = 0; q < kMaxBatch; q++)
                 if (q < np_) {
@@ -493,6 +525,217 @@ __global__ void __launch_bounds__(kColThreads, 1)
                 }
         }
         __syncthreads();   // the next batch overwrites the staged rows (and perhaps the inverse)
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Whole coloured sweeps in one launch.
+//
+// A colour step of a level with about one batch per SM is a chain of dependent
+// loads (batch, patch, DOFs, row ranges, entries, x) and a 1.6 k-cycle FP64 chain
+// (the inverse row), launched 2 x colours times per smoothing: 12 us per step
+// with k_schwarz_colour (9.5 since inverse_row), 6.5 here at 64 x 64 cells.  Only the x gather, the products and the x update depend
+// on the previous colour.  k_schwarz_sweep runs all steps of `runs` smoothings in
+// one cooperative launch of at most one CTA per SM: a CTA that has stored its x
+// arrives at the grid barrier and, before it waits, fetches the next colour's
+// rows -- DOF and row range from a flat table, up to kSwPre entries of its row
+// into registers, the right-hand side -- and starts the copy of the next inverse
+// into shared memory when it differs.  After the barrier come the x gather (L2;
+// other CTAs wrote x in this launch), the residual sums, the product, the update.
+// The sums are those of residual_rows and k_schwarz_colour in the same order:
+// the same bits.
+//
+// The barrier is a counter in global memory that every CTA increments once per
+// step; the wait is bounded (about a second), after which the CTA sets the error
+// word, writes NaN into one of its x entries (the caller's iteration then reports
+// a non-finite value) and leaves; a set error word makes later launches do the
+// same at once.  The last CTA to leave re-arms the counters.
+// ---------------------------------------------------------------------------
+constexpr int kSwMaxColours = 16;
+constexpr int kSwPre = kRowUnroll;            // prefetched entries per lane (kRowLanes lanes per row)
+constexpr int kSwThreads = 672;               // 96 registers, 168 rows per pass; patches up to this size
+
+struct SweepParams {
+    int ncol, runs, rounds;
+};
+
+__global__ void k_sweep_rows(int nb, const int* __restrict__ bpat, const int* __restrict__ bptr,
+                             const SchwarzImpl::BatchDesc* __restrict__ bd, const int64_t* __restrict__ pptr,
+                             const int* __restrict__ dofs, const int* __restrict__ rp, int4* __restrict__ brow)
+{
+    const SchwarzImpl::BatchDesc d = bd[blockIdx.x];
+    const int q0 = bptr[blockIdx.x];
+    (void)nb;
+    for (int k = threadIdx.x; k < d.np * d.m; k += blockDim.x) {
+        const int g = dofs[pptr[bpat[q0 + k / d.m]] + k % d.m];
+        brow[d.row0 + k] = make_int4(g, rp[g], rp[g + 1], 0);
+    }
+}
+
+template <typename T, typename IT, bool SM>
+__global__ void __launch_bounds__(kSwThreads, 1)
+    k_schwarz_sweep(const __grid_constant__ SweepParams P, CsrView A, const SchwarzImpl::BatchDesc* __restrict__ bd,
+                    const int* __restrict__ bslot, const int4* __restrict__ brow, const IT* __restrict__ inv, int mcap,
+                    int rows_cap,
+                    const T* __restrict__ b, T* x, double om, unsigned* bar, const int* done)
+{
+    if (done && *done) return;                                     // the same answer on every CTA
+    extern __shared__ __align__(16) unsigned char col_smem[];
+    // this CTA's first batch of every colour (np = 0: none); the last entry: a later round's
+    __shared__ SchwarzImpl::BatchDesc sbd[kSwMaxColours + 1];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x, G = (int)gridDim.x;
+    const int sub = tid & (kRowLanes - 1), li = tid / kRowLanes;   // residual role: lane of row li
+    constexpr int kPass = kSwThreads / kRowLanes;
+    IT* sAt = reinterpret_cast<IT*>(col_smem);
+    double* sr = reinterpret_cast<double*>(col_smem + (SM ? col_smem_inv<IT>(mcap) : 0));   // residuals of the batch rows
+    int* sg = reinterpret_cast<int*>(sr + rows_cap);               // their DOFs
+    auto batch_of = [&](int col, int round) { return __ldg(bslot + ((size_t)col * P.rounds + round) * G + blockIdx.x); };
+    if (tid < P.ncol) {
+        const int k = batch_of(tid, 0);
+        if (k >= 0)
+            sbd[tid] = bd[k];
+        else
+            sbd[tid].np = 0;
+    }
+    if (tid == 0) s_ok = *reinterpret_cast<volatile unsigned*>(bar + 2) == 0;
+    __syncthreads();
+    int64_t loaded = -1;                                           // the inverse in shared memory
+    // state fetched ahead of the barrier: the residual row's entries, its right-hand side, DOF
+    int c[kSwPre], k0 = 0, k1 = 0;
+    double v[kSwPre], bv = 0.0;
+    auto load_inverse = [&](const SchwarzImpl::BatchDesc& d) {
+        if (SM && d.off != loaded) {
+            const size_t bytes = (size_t)d.m * d.m * sizeof(IT);
+            const unsigned char* src = reinterpret_cast<const unsigned char*>(inv + d.off);
+            unsigned char* dst = reinterpret_cast<unsigned char*>(sAt);
+            const int g = ((reinterpret_cast<uintptr_t>(src) | bytes) & 15) == 0 ? 16 : (int)sizeof(IT);
+            if (tid < kSwThreads - 32)
+#pragma unroll 1
+                for (int k = tid * g; k < (int)bytes; k += (kSwThreads - 32) * g)
+                    cp_async_bytes(dst + k, src + k, g);
+            loaded = d.off;
+        }
+        cp_async_commit();
+    };
+    auto fetch = [&](const SchwarzImpl::BatchDesc& d, int i) {     // row i of the batch: entries and right-hand side
+        k0 = k1 = 0;
+        if (i < d.np * d.m) {
+            const int4 r = __ldg(brow + d.row0 + i);
+            k0 = r.y + sub;
+            k1 = r.z;
+            if (sub == 0) {
+                bv = (double)__ldg(b + r.x);
+                sg[i] = r.x;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kSwPre; u++) {
+            const int k = k0 + u * kRowLanes;
+            c[u] = k < k1 ? __ldg(A.col + k) : -1;
+            v[u] = k < k1 ? __ldg(A.val + k) : 0.0;
+        }
+    };
+    auto process = [&](const SchwarzImpl::BatchDesc& d, bool cold) {   // rows 0 .. kPass - 1 fetched unless cold
+        const int m = d.m, np_ = d.np, rows = np_ * m;
+#pragma unroll 1
+        for (int i0 = 0; i0 < rows; i0 += kPass) {
+            if (i0 || cold) fetch(d, i0 + li);
+            double acc = 0.0;
+            T xv[kSwPre];
+#pragma unroll
+            for (int u = 0; u < kSwPre; u++) xv[u] = c[u] >= 0 ? __ldcg(x + c[u]) : (T)0;
+#pragma unroll
+            for (int u = 0; u < kSwPre; u++)
+                if (c[u] >= 0) acc += v[u] * (double)xv[u];
+#pragma unroll 1
+            for (int k = k0 + kSwPre * kRowLanes; k < k1; k += kRowLanes)
+                acc += __ldg(A.val + k) * (double)__ldcg(x + __ldg(A.col + k));
+#pragma unroll
+            for (int o = 1; o < kRowLanes; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (i0 + li < rows && sub == 0) sr[i0 + li] = bv - acc;
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        double xg[kMaxBatch];                                      // the entries to be updated: loads in flight during the product
+#pragma unroll
+        for (int q = 0; q < kMaxBatch; q++) xg[q] = tid < m && q < np_ ? (double)__ldcg(x + sg[q * m + tid]) : 0.0;
+        const IT* Ag = inv + d.off;
+        if (const int i = tid; i < m) {                            // m <= kSwThreads
+            double acc[kMaxBatch];
+            inverse_row(np_, m, sr, [&](int j) { return SM ? (double)sAt[j * m + i] : (double)__ldg(Ag + (size_t)j * m + i); },
+                        acc);
+#pragma unroll
+            for (int q = 0; q < kMaxBatch; q++)
+                if (q < np_) x[sg[q * m + i]] = (T)(xg[q] + acc[q] * om);
+        }
+        __syncthreads();                                           // sr and the inverse are free again
+    };
+    auto colour_of = [&](int s) {                                  // forward, backward, forward, ...
+        const int r = s % (2 * P.ncol);
+        return r < P.ncol ? r : 2 * P.ncol - 1 - r;
+    };
+    const int steps = 2 * P.ncol * P.runs;
+    bool ok = s_ok != 0;
+    // step -1 only fetches for step 0 (one code path: registers are what this kernel is short of)
+#pragma unroll 1
+    for (int s = -1; ok && s < steps; s++) {
+        if (s >= 0) {
+            const int col = colour_of(s);
+#pragma unroll 1
+            for (int round = 0; round < P.rounds; round++) {       // more batches than CTAs: several rounds
+                if (round) {
+                    const int k = batch_of(col, round);
+                    if (k < 0) break;
+                    if (tid == 0) sbd[kSwMaxColours] = bd[k];
+                    __syncthreads();
+                    load_inverse(sbd[kSwMaxColours]);
+                }
+                const SchwarzImpl::BatchDesc& d = sbd[round ? kSwMaxColours : col];
+                if (!d.np) break;
+                process(d, round != 0);
+            }
+        }
+        if (s + 1 == steps) break;
+        // the last warp, which has few residual rows or none on patches of up to 168 DOFs,
+        // meets the other CTAs while the rest fetch
+        if (tid == kSwThreads - 1 && s >= 0) {
+            // this CTA's x (behind process's barrier) is out before the arrival
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        }
+        const SchwarzImpl::BatchDesc& nx = sbd[colour_of(s + 1)];
+        if (nx.np) {
+            fetch(nx, li);
+            load_inverse(nx);
+        }
+        if (s < 0) continue;
+        if (tid == kSwThreads - 1) {
+            const unsigned want = (unsigned)(s + 1) * (unsigned)G;
+            bool in = false;
+#pragma unroll 1
+            for (int i = 0; i < (1 << 21) && !in; i++) {
+                unsigned now;
+                asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
+                in = now >= want;
+                if (!in && i > 64) __nanosleep(64);
+            }
+            s_ok = in;
+        }
+        __syncthreads();
+        ok = s_ok != 0;
+    }
+    cp_async_wait<0>();
+    if (tid == 0) {
+        if (!ok) {
+            atomicOr(bar + 2, 1u);
+            x[brow[0].x] = (T)NAN;
+        }
+        __threadfence();
+        if (atomicAdd(bar + 1, 1u) == (unsigned)G - 1u) {          // the last CTA: nobody waits any more
+            bar[0] = 0;
+            bar[1] = 0;
+            __threadfence();
+        }
     }
 }
 
@@ -810,6 +1053,7 @@ void SchwarzImpl::init(Context* ctx, Matrix* Am, int kind_, double omega_, int n
             bptr.alloc(h_bptr.size());
             JFG_CUDA(cudaMemcpyAsync(bpat.p, h_bpat.data(), sizeof(int) * h_bpat.size(), cudaMemcpyHostToDevice, st));
             JFG_CUDA(cudaMemcpyAsync(bptr.p, h_bptr.data(), sizeof(int) * h_bptr.size(), cudaMemcpyHostToDevice, st));
+            plan_sweep(h_bpat, h_bptr, hp, hoff2, st);
         }
         // ColoredMultiplicativeSubspaceCorrection.solve starts with patch 0 alone
         int zero = 0;
@@ -838,6 +1082,104 @@ void SchwarzImpl::init(Context* ctx, Matrix* Am, int kind_, double omega_, int n
                                  st));
     }
     JFG_CUDA(cudaStreamSynchronize(st));
+}
+
+// Whole sweeps in one launch where every colour runs on k_schwarz_colour (2) or
+// every one on its global-memory variant (3): about one batch per SM and colour,
+// so the steps are latency, not work.  Colours of k_schwarz_batch (many more
+// patches than SMs) keep their launches: 4 small CTAs per SM hide more there.
+// JFEM_SCHWARZ_SWEEP=0 keeps one launch per colour.
+void SchwarzImpl::plan_sweep(const std::vector<int>& h_bpat, const std::vector<int>& h_bptr,
+                             const std::vector<int64_t>& hp, const std::vector<int64_t>& hoff, cudaStream_t st)
+{
+    const char* e = getenv("JFEM_SCHWARZ_SWEEP");
+    if ((e && e[0] == '0') || colours.empty() || colours.size() > (size_t)kSwMaxColours) return;
+    int kern = 0, most = 0;
+    for (const auto& col : colours) {
+        if (col.count == 0) continue;
+        if (col.kern < 2 || (kern && col.kern != kern)) return;
+        kern = col.kern;
+        most = std::max(most, col.b_count);
+        sweep_mcap = std::max(sweep_mcap, col.mcap);
+        sweep_rows = std::max(sweep_rows, col.rows_cap);
+    }
+    if (!kern || sweep_mcap > kSwThreads) return;
+    sweep_smem = kern == 2;
+    if ((sweep_smem ? col_smem_inv<double>(sweep_mcap) : 0) + (size_t)sweep_rows * 12 > kColSmemMax) return;
+    int dev = 0, coop = 0, nsm = 0;
+    JFG_CUDA(cudaGetDevice(&dev));
+    JFG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    JFG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    if (!coop) return;
+    std::vector<BatchDesc> d(h_bptr.size(), BatchDesc{0, 1, 0, 0, 0});
+    int row0 = 0;
+    for (const auto& col : colours)
+        for (int q = 0; q < col.b_count; q++) {
+            const int k = col.b_start + q, p0 = h_bpat[h_bptr[k]];
+            const int m = (int)(hp[p0 + 1] - hp[p0]), np_ = h_bptr[k + 1] - h_bptr[k];
+            d[k] = BatchDesc{hoff[p0], m, np_, row0, 0};
+            JFG_CHECK((int64_t)row0 + (int64_t)m * np_ < INT32_MAX, JFG_ERR_UNSUPPORTED, "too many patch rows");
+            row0 += m * np_;
+        }
+    // A CTA keeps the inverse of its last batch in shared memory, and every step
+    // waits for the slowest CTA: a batch goes to a CTA that has its inverse, else
+    // to a new CTA while there are SMs, else to the one idle for longest.
+    sweep_rounds = std::max(1, (most + nsm - 1) / nsm);
+    std::vector<std::vector<int>> slot(colours.size());
+    int grid = std::min(most, nsm);
+    if (sweep_rounds == 1) {
+        std::vector<int64_t> held;
+        std::vector<int> last;
+        for (size_t c = 0; c < colours.size(); c++) {
+            std::vector<int> own(nsm, -1), todo;
+            auto give = [&](int k, int b) {
+                own[b] = k;
+                held[b] = d[k].off;
+                last[b] = (int)c;
+            };
+            for (int q = 0; q < colours[c].b_count; q++) {
+                const int k = colours[c].b_start + q;
+                int b = 0;
+                while (b < (int)held.size() && (own[b] >= 0 || held[b] != d[k].off)) b++;
+                if (b < (int)held.size())
+                    give(k, b);
+                else
+                    todo.push_back(k);
+            }
+            for (int k : todo) {
+                int b = -1;
+                if ((int)held.size() < nsm) {
+                    b = (int)held.size();
+                    held.push_back(-1);
+                    last.push_back(-1);
+                } else {
+                    for (int t = 0; t < nsm; t++)
+                        if (own[t] < 0 && (b < 0 || last[t] < last[b])) b = t;
+                }
+                give(k, b);
+            }
+            slot[c] = own;
+        }
+        grid = (int)held.size();
+    }
+    std::vector<int> hs(colours.size() * (size_t)sweep_rounds * grid, -1);
+    for (size_t c = 0; c < colours.size(); c++)
+        for (int k = 0; k < sweep_rounds * grid; k++)
+            hs[c * (size_t)sweep_rounds * grid + k] =
+                sweep_rounds == 1 ? slot[c][k] : (k < colours[c].b_count ? colours[c].b_start + k : -1);
+    bslot.alloc(hs.size());
+    JFG_CUDA(cudaMemcpyAsync(bslot.p, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice, st));
+    bdesc.alloc(d.size());
+    brow.alloc((size_t)row0);
+    bar.alloc(4);
+    JFG_CUDA(cudaMemsetAsync(bar.p, 0, 4 * sizeof(unsigned), st));
+    JFG_CUDA(cudaMemcpyAsync(bdesc.p, d.data(), sizeof(BatchDesc) * d.size(), cudaMemcpyHostToDevice, st));
+    k_sweep_rows<<<(unsigned)d.size(), 256, 0, st>>>((int)d.size(), bpat.p, bptr.p, bdesc.p, pptr.p, dofs.p,
+                                                    A->csr_ptr.p, brow.p);
+    JFG_CUDA(cudaGetLastError());
+    note_launch();
+    JFG_CUDA(cudaStreamSynchronize(st));
+    sweep_grid = grid;
 }
 
 const float* SchwarzImpl::inverses32()
@@ -921,11 +1263,46 @@ void SchwarzImpl::colour_step(const Colour& col, const T* b, T* x, double om, co
 }
 
 template <typename T>
+void SchwarzImpl::sweep(int runs, const T* b, T* x, const int* done, cudaStream_t st)
+{
+    using IT = T;
+    const IT* iv = static_cast<const IT*>(inv_of<T>(this));
+    SweepParams P = {};
+    P.runs = runs;
+    P.ncol = (int)colours.size();
+    P.rounds = sweep_rounds;
+    auto* kern = sweep_smem ? k_schwarz_sweep<T, IT, true> : k_schwarz_sweep<T, IT, false>;
+    static bool attr = false;          // per instantiation
+    if (!attr) {
+        JFG_CUDA(cudaFuncSetAttribute(k_schwarz_sweep<T, IT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kColSmemMax));
+        JFG_CUDA(cudaFuncSetAttribute(k_schwarz_sweep<T, IT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kColSmemMax));
+        attr = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)sweep_grid);
+    cfg.blockDim = dim3(kSwThreads);
+    cfg.dynamicSmemBytes = (sweep_smem ? col_smem_inv<IT>(sweep_mcap) : 0) + (size_t)sweep_rows * 12;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    JFG_CUDA(cudaLaunchKernelEx(&cfg, kern, P, csr_of(A), (const BatchDesc*)bdesc.p, (const int*)bslot.p,
+                                (const int4*)brow.p, iv, sweep_mcap, sweep_rows, b, x, omega, bar.p, done));
+    note_launch();
+}
+
+template <typename T>
 void SchwarzImpl::apply(const T* b, T* x, const Scratch&, const int* done, cudaStream_t st)
 {
     using IT = T;
     const IT* iv = static_cast<const IT*>(inv_of<T>(this));
-    if (kind == JFG_SCHWARZ_MULTIPLICATIVE) {
+    if (sweep_grid) {
+        sweep<T>(1, b, x, done, st);
+    } else if (kind == JFG_SCHWARZ_MULTIPLICATIVE) {
         // MultiplicativeSubspaceCorrection.apply: patches forward, then backward
         k_schwarz_seq<T, IT><<<1, kSchThreads, 0, st>>>(csr_of(A), seq.p, 2 * np, pptr.p, dofs.p, inv_off.p, iv, b, x,
                                                         done);

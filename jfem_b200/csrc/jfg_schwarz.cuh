@@ -37,6 +37,20 @@ struct SchwarzImpl {
     DevBuf<double> lsol;                // local solutions of the patches of one sweep step
     DevBuf<int> flag;
     DevBuf<int> bpat, bptr;             // batches of patches sharing an inverse (colours with many patches)
+    // whole sweeps in one cooperative launch (k_schwarz_sweep): per batch its
+    // descriptor and per batch row (DOF, first entry, end of entries)
+    struct BatchDesc {
+        int64_t off;                    // inverse
+        int m, np, row0, pad;           // patch size, patches, first row of the row table
+    };
+    DevBuf<BatchDesc> bdesc;
+    DevBuf<int4> brow;
+    DevBuf<unsigned> bar;               // arrivals, exits, error
+    DevBuf<int> bslot;                  // per colour sweep_rounds x sweep_grid: the batch of a CTA, or -1
+    int sweep_rounds = 1;
+    int sweep_grid = 0;                 // CTAs of k_schwarz_sweep (0: one launch per colour)
+    int sweep_mcap = 0, sweep_rows = 0; // largest patch and batch rows of the sweep's colours
+    bool sweep_smem = false;            // the inverses fit shared memory
     struct Colour {
         int start = 0, count = 0;       // range of cpat
         bool independent = false;       // patches neither share nor couple DOFs: one fused kernel
@@ -63,11 +77,19 @@ struct SchwarzImpl {
     template <typename T>
     void smooth(int runs, const T* b, T* x, const Scratch& sc, const int* done, cudaStream_t st)
     {
+        if (sweep_grid && runs > 0) {
+            sweep<T>(runs, b, x, done, st);
+            return;
+        }
         for (int i = 0; i < runs; i++) apply<T>(b, x, sc, done, st);
     }
     const float* inverses32();
 
 private:
+    void plan_sweep(const std::vector<int>& h_bpat, const std::vector<int>& h_bptr, const std::vector<int64_t>& hp,
+                    const std::vector<int64_t>& hoff, cudaStream_t st);
+    template <typename T>
+    void sweep(int runs, const T* b, T* x, const int* done, cudaStream_t st);
     template <typename T>
     void colour_step(const Colour& col, const T* b, T* x, double om, const int* done, cudaStream_t st);
     void build_scatter(Colour& col, const std::vector<int64_t>& hp, const std::vector<int>& hd,
