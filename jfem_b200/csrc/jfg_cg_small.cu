@@ -1,12 +1,13 @@
 // Unpreconditioned CG (IterativeSolver.solveCG, IterativeSolver.java:48-103)
 // for small systems in one launch: one 8-CTA thread-block cluster runs every
 // iteration.  Each thread owns up to two rows and keeps their x, r, p and A p
-// entries in registers; p is also written to global memory for the other
-// rows' products; the two dot products of an iteration are reduced through
+// entries in registers; the two dot products of an iteration are reduced through
 // distributed shared memory (every CTA sums the eight CTA partials in rank
 // order, so every thread holds the same value and takes the same branch).
-// Three cluster barriers per iteration replace the ~5 kernel launches of the
-// graph-captured loop, whose launch latency dominates at this size.  The
+// Two cluster barriers per iteration with the matrix in shared memory
+// (k_cg_small_smem), three with p in global memory (k_cg_small), replace the ~5
+// kernel launches of the graph-captured loop, whose launch latency dominates at
+// this size.  The
 // scalar recurrences and the stopping test are those of the multi-kernel CG
 // (alpha = rz / p.Ap, beta = rr' / rr, `iter < maxit && ||r|| > tol`,
 // NONFINITE on a non-finite residual); the loop is bounded by maxit.
@@ -28,6 +29,7 @@ constexpr int kCgThreads = 1024;
 constexpr int kCgRowsPerThread = 2;
 constexpr int kSmThreads = 512;      // shared-memory variant: 512 threads x 4 rows
 constexpr int kSmRows = 4;
+constexpr int kSmMaxRows = 2048;     // rows per CTA of the shared-memory variant
 
 struct CgSmallArgs {
     int n;
@@ -179,46 +181,99 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads, 1)
     cl.sync();      // no CTA leaves while another may still read its shared memory
 }
 
-// The same iteration with the matrix rows and a replica of p in shared
-// memory: CTA q owns the contiguous rows [q R, (q + 1) R) and keeps their CSR
-// slice; every thread stores the new p of its rows into all eight CTAs'
-// replicas (DSMEM stores) before the barrier, so the products read only
-// shared memory.  Used when the slice and the replica fit one CTA's shared
-// memory.
-struct CgSmemLayout {
-    int R;              // rows per CTA
-    int max_nnz;        // largest CSR slice of a CTA
-    size_t bytes;       // dynamic shared memory per CTA
+// The same iteration with the matrix rows in shared memory: CTA q owns the
+// contiguous rows [q R, (q + 1) R), keeps their CSR slice and the window [lo, hi)
+// of p and r that the slice's columns (and its own rows) span.  Every thread
+// stores the new r of its rows into the windows that hold them (DSMEM stores),
+// before the barrier of the ||r||^2 sum; each CTA then updates p = r + p beta over
+// its own window, the arithmetic of the row's owner, so no barrier separates the
+// direction update from the next product: two cluster barriers per iteration.  A
+// sum is one push per CTA into a slot of every other, then eight local loads in
+// rank order.  Bound by those two rounds (~1,400 cycles each); with p itself
+// broadcast to all CTAs, a third barrier for it and sums read remotely, an
+// iteration at 4,225 rows took 5.2 us.  Used when slice and windows fit.
+struct CgRange {
+    int nnz, lo, hi;    // CSR slice and window of a CTA
+};
+struct CgWindows {
+    CgRange c[kCgCtas];
 };
 
+__global__ void __launch_bounds__(256) k_cg_small_range(int n, int R, const int* __restrict__ ptr,
+                                                        const int* __restrict__ col, CgRange* __restrict__ out)
+{
+    __shared__ int slo[8], shi[8];
+    const int r0 = min(n, (int)blockIdx.x * R), r1 = min(n, r0 + R);
+    int lo = r0, hi = r1;
+    for (int k = ptr[r0] + threadIdx.x; k < ptr[r1]; k += 256) {
+        lo = min(lo, col[k]);
+        hi = max(hi, col[k] + 1);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        slo[threadIdx.x >> 5] = lo;
+        shi[threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) {
+            lo = min(lo, slo[w]);
+            hi = max(hi, shi[w]);
+        }
+        out[blockIdx.x] = CgRange{ptr[r1] - ptr[r0], lo, hi};
+    }
+}
+
+// cluster_sum with the partials pushed: the same sums in the same order; slot[kCgCtas] has one call site
+__device__ __forceinline__ double pushed_sum(cg::cluster_group& cl, double v, double* warp_part, double* slot)
+{
+    v = warp_sum(v);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) warp_part[w] = v;
+    __syncthreads();
+    if (w == 0) {                                             // the CTA's warps in order, by every lane that pushes
+        v = 0.0;
+#pragma unroll
+        for (int i = 0; i < kSmThreads / 32; i++) v += warp_part[i];
+        if (l < kCgCtas) *cl.map_shared_rank(slot + cl.block_rank(), l) = v;
+    }
+    cl.sync();
+    double t = 0.0;
+#pragma unroll
+    for (int r = 0; r < kCgCtas; r++) t += slot[r];
+    return t;
+}
+
 __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
-    k_cg_small_smem(CgSmallArgs a, int R, int max_nnz)
+    k_cg_small_smem(CgSmallArgs a, const __grid_constant__ CgWindows win, int R, int max_nnz, int max_win)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double warp_part[kSmThreads / 32];
-    __shared__ double slots[2];
-    double* p_all = reinterpret_cast<double*>(smem);                       // n
-    double* lval = p_all + a.n;                                            // max_nnz
+    __shared__ double slot_pap[kCgCtas], slot_rr[kCgCtas];
+    double* pw = reinterpret_cast<double*>(smem);                          // max_win
+    double* rw = pw + max_win;                                             // max_win
+    double* lval = rw + max_win;                                           // max_nnz
     int* lptr = reinterpret_cast<int*>(lval + max_nnz);                    // R + 1
     int* lcol = lptr + R + 1;                                              // max_nnz
     cg::cluster_group cl = cg::this_cluster();
     const int q = (int)cl.block_rank();
-    const int r0 = q * R, r1 = min(a.n, r0 + R);
-    const int nr = r1 > r0 ? r1 - r0 : 0;
+    const int r0 = min(a.n, q * R), r1 = min(a.n, r0 + R), nr = r1 - r0;
+    const int lo = win.c[q].lo, W = win.c[q].hi - lo;
     const bool lead = q == 0 && threadIdx.x == 0;
     Ctl* c = a.ctl;
     const double tol = c->tol;
     const int maxit = c->maxit;
     double* hist = c->hist;
     const int hist_cap = c->hist_cap;
-    // the CTA's CSR slice, with row pointers relative to its first entry
-    const int e0 = nr ? a.ptr[r0] : 0;
-    const int ne = nr ? a.ptr[r1] - e0 : 0;
+    // the CTA's CSR slice, row pointers relative to its first entry, columns to the window
+    const int e0 = a.ptr[r0], ne = a.ptr[r1] - e0;
     for (int i = threadIdx.x; i <= nr; i += kSmThreads) lptr[i] = a.ptr[r0 + i] - e0;
     for (int k = threadIdx.x; k < ne; k += kSmThreads) {
-        lcol[k] = a.col[e0 + k];
+        lcol[k] = a.col[e0 + k] - lo;
         lval[k] = a.val[e0 + k];
     }
+    for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = a.x[lo + i];      // x0, for the first residual
     int rows[kSmRows];
     double x[kSmRows], r[kSmRows], p[kSmRows], ap[kSmRows];
 #pragma unroll
@@ -227,46 +282,64 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
         x[j] = r[j] = p[j] = ap[j] = 0.0;
         if (rows[j] < nr) x[j] = a.x[r0 + rows[j]];
     }
-    __syncthreads();
-    auto local_dot = [&](int lr, const double* v) {
+    cl.sync();                                                // every CTA runs before a store reaches it
+    auto local_dot = [&](int lr) {                            // five entries loaded at a time, summed in order
         double s = 0.0;
-        for (int k = lptr[lr]; k < lptr[lr + 1]; k++) s += lval[k] * v[lcol[k]];
+        const int k1 = lptr[lr + 1];
+        for (int k = lptr[lr]; k < k1; k += 5) {
+            int cc[5];
+            double v[5];
+#pragma unroll
+            for (int u = 0; u < 5; u++) {
+                cc[u] = k + u < k1 ? lcol[k + u] : 0;
+                v[u] = k + u < k1 ? lval[k + u] : 0.0;
+            }
+            double pv[5];
+#pragma unroll
+            for (int u = 0; u < 5; u++) pv[u] = pw[cc[u]];
+#pragma unroll
+            for (int u = 0; u < 5; u++)
+                if (k + u < k1) s += v[u] * pv[u];
+        }
         return s;
     };
-    // r = b - A x0 (x0 read from global once), rr
+    auto push_r = [&]() {
+#pragma unroll
+        for (int j = 0; j < kSmRows; j++)
+            if (rows[j] < nr) {
+                const int g = r0 + rows[j];
+#pragma unroll
+                for (int t = 0; t < kCgCtas; t++)
+                    if (g >= win.c[t].lo && g < win.c[t].hi) *cl.map_shared_rank(rw + (g - win.c[t].lo), t) = r[j];
+            }
+    };
+    // r = b - A x0, rr
     double part = 0.0;
 #pragma unroll
     for (int j = 0; j < kSmRows; j++)
         if (rows[j] < nr) {
-            double s = 0.0;
-            for (int k = lptr[rows[j]]; k < lptr[rows[j] + 1]; k++) s += lval[k] * a.x[lcol[k]];
-            r[j] = a.b[r0 + rows[j]] - s;
+            r[j] = a.b[r0 + rows[j]] - local_dot(rows[j]);
             part += r[j] * r[j];
         }
-    double rr = cluster_sum<kSmThreads>(cl, part, warp_part, &slots[0]);
+    push_r();
+    double rr = pushed_sum(cl, part, warp_part, slot_rr);
     double rz = rr;
     int iter = 0, status = JFG_NOT_CONVERGED, not_pd = 0;
     double res = sqrt(rr);
     bool done = stop_test(c, res, iter, maxit, tol, &status);
-    auto broadcast_p = [&]() {
-#pragma unroll
-        for (int j = 0; j < kSmRows; j++)
-            if (rows[j] < nr)
-                for (int t = 0; t < kCgCtas; t++) *cl.map_shared_rank(p_all + r0 + rows[j], t) = p[j];
-    };
 #pragma unroll
     for (int j = 0; j < kSmRows; j++) p[j] = r[j];
-    broadcast_p();
-    cl.sync();
+    for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i];
+    __syncthreads();
     while (!done) {
         part = 0.0;
 #pragma unroll
         for (int j = 0; j < kSmRows; j++)
             if (rows[j] < nr) {
-                ap[j] = local_dot(rows[j], p_all);
+                ap[j] = local_dot(rows[j]);
                 part += p[j] * ap[j];
             }
-        const double pap = cluster_sum<kSmThreads>(cl, part, warp_part, &slots[1]);
+        const double pap = pushed_sum(cl, part, warp_part, slot_pap);
         const double alpha = rz / pap;
         if (!(pap > 0)) not_pd = 1;
         part = 0.0;
@@ -277,7 +350,8 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
                 r[j] = r[j] - ap[j] * alpha;
                 part += r[j] * r[j];
             }
-        const double rr_new = cluster_sum<kSmThreads>(cl, part, warp_part, &slots[0]);
+        push_r();
+        const double rr_new = pushed_sum(cl, part, warp_part, slot_rr);
         iter++;
         const double beta = rr_new / rr;
         rz = rr_new;
@@ -289,8 +363,8 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
 #pragma unroll
         for (int j = 0; j < kSmRows; j++)
             if (rows[j] < nr) p[j] = r[j] + p[j] * beta;
-        broadcast_p();
-        cl.sync();
+        for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i] + pw[i] * beta;
+        __syncthreads();
     }
 #pragma unroll
     for (int j = 0; j < kSmRows; j++)
@@ -304,7 +378,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
         c->not_pd = not_pd;
         c->done = 1;
     }
-    cl.sync();      // no CTA leaves while another may still read or write its shared memory
+    cl.sync();      // no CTA leaves while another may still write its shared memory
 }
 
 }  // namespace
@@ -323,24 +397,30 @@ void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
     const int n = A->rows;
     w.v64[0].alloc((size_t)n);
     CgSmallArgs a{n, A->csr_ptr.p, A->csr_col.p, A->csr_val.p, b, x, w.v64[0].p, w.ctl.p};
-    // shared-memory variant when a CTA's CSR slice and the p replica fit
+    // shared-memory variant when a CTA's CSR slice and its windows of p and r fit
     const int R = (n + kCgCtas - 1) / kCgCtas;
-    if (A->cg_small_nnz < 0) {      // once per matrix: the largest row block's CSR slice
-        std::vector<int> ptr((size_t)n + 1);
-        JFG_CUDA(cudaMemcpyAsync(ptr.data(), A->csr_ptr.p, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, st));
+    if (A->cg_small_win.size() != kCgCtas * 3) {      // once per matrix: slices and windows of the row blocks
+        DevBuf<CgRange> d;
+        d.alloc(kCgCtas);
+        k_cg_small_range<<<kCgCtas, 256, 0, st>>>(n, R, A->csr_ptr.p, A->csr_col.p, d.p);
+        JFG_CUDA(cudaGetLastError());
+        note_launch();
+        A->cg_small_win.resize(kCgCtas * 3);
+        static_assert(sizeof(CgRange) == 3 * sizeof(int), "three ints per row block");
+        JFG_CUDA(cudaMemcpyAsync(A->cg_small_win.data(), d.p, sizeof(CgRange) * kCgCtas, cudaMemcpyDeviceToHost, st));
         JFG_CUDA(cudaStreamSynchronize(st));
-        int mx = 0;
-        for (int q = 0; q < kCgCtas; q++) {
-            const int r0 = std::min(n, q * R), r1 = std::min(n, r0 + R);
-            mx = std::max(mx, ptr[r1] - ptr[r0]);
-        }
-        A->cg_small_nnz = mx;
     }
-    const int max_nnz = A->cg_small_nnz;
-    const size_t bytes = sizeof(double) * ((size_t)n + max_nnz) + sizeof(int) * ((size_t)R + 1 + max_nnz) + 16;
+    CgWindows win;
+    int max_nnz = 0, max_win = 0;
+    for (int q = 0; q < kCgCtas; q++) {
+        win.c[q] = CgRange{A->cg_small_win[3 * q], A->cg_small_win[3 * q + 1], A->cg_small_win[3 * q + 2]};
+        max_nnz = std::max(max_nnz, win.c[q].nnz);
+        max_win = std::max(max_win, win.c[q].hi - win.c[q].lo);
+    }
+    const size_t bytes = sizeof(double) * (2 * (size_t)max_win + max_nnz) + sizeof(int) * ((size_t)R + 1 + max_nnz) + 16;
     constexpr size_t kSmemCap = (size_t)200 * 1024;
     const char* e = getenv("JFEM_SMALL_CG_SMEM");
-    const bool smem_ok = !(e && e[0] == '0') && R <= kSmThreads * kSmRows && bytes <= kSmemCap;
+    const bool smem_ok = !(e && e[0] == '0') && R <= kSmMaxRows && bytes <= kSmemCap;
     if (smem_ok) {
         static int attr_dev = -1;     // the opt-in shared memory size, set once per device
         int dev = 0;
@@ -349,7 +429,7 @@ void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
             JFG_CUDA(cudaFuncSetAttribute(k_cg_small_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
             attr_dev = dev;
         }
-        k_cg_small_smem<<<kCgCtas, kSmThreads, bytes, st>>>(a, R, max_nnz);
+        k_cg_small_smem<<<kCgCtas, kSmThreads, bytes, st>>>(a, win, R, max_nnz, max_win);
     } else {
         k_cg_small<<<kCgCtas, kCgThreads, 0, st>>>(a);
     }

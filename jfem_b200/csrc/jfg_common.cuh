@@ -161,7 +161,7 @@ struct Matrix {
     DevBuf<float> st_val32;
     DevBuf<__nv_bfloat16> st_val16;
     DevBuf<__half> st_valh;
-    int cg_small_nnz = -1;        // small-system CG: largest CSR slice of its 8 row blocks (-1: not computed)
+    std::vector<int> cg_small_win; // small-system CG: CSR slice and column window of its 8 row blocks (empty: not computed)
     Matrix* transposed = nullptr; // lazily built for tvMul
     uint64_t uid = 0;             // unique id (keys of cached CUDA graphs)
     Matrix();
