@@ -139,8 +139,10 @@ int jfg_destroy(jfg_ctx* ctx)
     cudaSetDevice(ctx->c.device);
     cudaStreamSynchronize(ctx->c.stream);
     cudaStream_t s = ctx->c.stream;
+    const int dev = ctx->c.device;
     delete ctx;
     if (s) cudaStreamDestroy(s);
+    jfg::pool_trim(dev);
     return JFG_OK;
 }
 
@@ -162,6 +164,7 @@ int jfg_release_scratch(jfg_ctx* ctx)
         JFG_CUDA(cudaStreamSynchronize(ctx->c.stream));
         ctx->c.gemm_rows.release();
         ctx->c.gemm_ws.release();
+        jfg::pool_trim(ctx->c.device);
         return JFG_OK;
     });
 }

@@ -43,17 +43,24 @@ struct Error {
         if (!(cond)) throw ::jfg::Error{(code), (text)};                                   \
     } while (0)
 
+// device blocks kept between owners (jfg_pool.cu)
+void* pool_alloc(size_t bytes, int* dev);
+void pool_free(void* p, size_t bytes, int dev) noexcept;
+void pool_trim(int dev) noexcept;
+
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    int dev = 0;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
+    static size_t bytes(size_t count) { return (count ? count : 1) * sizeof(T); }
     void release()
     {
-        if (p) cudaFree(p);
+        if (p) pool_free(p, bytes(n), dev);
         p = nullptr;
         n = 0;
     }
@@ -61,7 +68,7 @@ struct DevBuf {
     {
         if (count <= n && p) return;
         release();
-        JFG_CUDA(cudaMalloc(&p, (count ? count : 1) * sizeof(T)));
+        p = static_cast<T*>(pool_alloc(bytes(count), &dev));
         n = count;
     }
 };
