@@ -262,7 +262,17 @@ __device__ __forceinline__ void tail_own(int R, int n, int c, F f)
     }
 }
 
-template <typename T>
+// FMG: fullVCycleCorrection on the levels 0..top instead of one V-cycle from a
+// zero guess.  The right-hand side of the top level is restricted down to
+// level 0 first, into the vectors b; then every level lt = 1..top starts from
+// the raw prolongation of level lt - 1's result and runs a V-cycle with the
+// right-hand side b, whose restrictions overwrite the b of the levels below
+// lt only: those levels have had their turn, so no vector is added.
+// Bound, as the V-cycle's tail, by the latency of its phases (0.3 us on one
+// CTA, 0.7-1 us over the cluster); as launches each phase costs 3.5-5 us.
+// Q1 224 x 224, FP64, full multigrid and 3 V-cycles: 105 launches and 430 us
+// -> 36 launches and 345 us an application, the same sums in a row's order.
+template <typename T, bool FMG>
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_constant__ TailParams<T> P)
 {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -291,63 +301,33 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
         T* b = vec(L.off_b);
         tail_own(L.Rl, L.n, c, [&](int t) { b[t] = P.b_top[c * L.Rl + t]; });
     }
-    __syncthreads();
-    for (int l = P.top; l >= 1; l--) {
-        const TailLevel<T>& L = P.lv[l];
+    // Jacobi sweeps k0..runs-1 of level l from the vector at cur_off, ending
+    // in x: sweeps before the last end a phase of level l, the last one a
+    // phase read next by a level that is local or not (loc_next)
+    auto sweeps = [&](const TailLevel<T>& L, int k0, int cur_off, bool loc_next) {
         const T* b = vec(L.off_b);
         const T* dinv = vec(L.off_dinv);
         const T om = L.omega;
-        // the first sweep from the zero guess lands where the last one ends in x
-        T* cur = vec((L.runs % 2 == 1) ? L.off_x : L.off_t);
-        int cur_off = (L.runs % 2 == 1) ? L.off_x : L.off_t;
-        const bool loc = L.local != 0;
-        if (l == P.top) {   // below the top the restriction phase did it
-            tail_own(L.Rl, L.n, c, [&](int t) { cur[t] = (T)0 + (dinv[t] * b[t]) * om; });
-            phase_end(loc);
-        }
-        for (int k = 1; k < L.runs; k++) {
+        for (int k = k0; k < L.runs; k++) {
             const int alt_off = cur_off == L.off_x ? L.off_t : L.off_x;
+            const T* cu = vec(cur_off);
             T* alt = vec(alt_off);
             TailMat A = L.A;
             A.xoff = cur_off;
-            const T* cu = cur;
             tail_spmv<T>(sm, A, c, [&](int t, T s) { alt[t] = cu[t] + (dinv[t] * (b[t] - s)) * om; });
-            phase_end(loc);
-            cur = alt;
+            const bool last = k == L.runs - 1 && alt_off == L.off_x;
+            phase_end(last ? loc_next : L.local != 0);
             cur_off = alt_off;
         }
-        {   // residual r = b - A x
-            T* r = vec(L.off_r);
-            TailMat A = L.A;
-            A.xoff = L.off_x;
-            tail_spmv<T>(sm, A, c, [&](int t, T s) { r[t] = b[t] - s; });
-            phase_end(loc);   // level l - 1 is local whenever level l is
+        if (cur_off != L.off_x) {
+            const T* cu = vec(cur_off);
+            T* x = vec(L.off_x);
+            tail_own(L.Rl, L.n, c, [&](int t) { x[t] = cu[t]; });
+            phase_end(loc_next);
         }
-        {   // restriction into level l - 1 with zero boundary values (and its fused first sweep)
-            const TailLevel<T>& Cl = P.lv[l - 1];
-            TailMat R = L.R;
-            R.xoff = L.off_r;
-            T* bc = vec(Cl.off_b);
-            const unsigned char* mask = sm + Cl.off_mask;
-            if (l - 1 >= 1) {
-                const T* dc = vec(Cl.off_dinv);
-                T* xd = vec((Cl.runs % 2 == 1) ? Cl.off_x : Cl.off_t);
-                const T oc = Cl.omega;
-                tail_spmv<T>(sm, R, c, [&](int t, T s) {
-                    const T v = mask[t] ? (T)0 : s;
-                    bc[t] = v;
-                    xd[t] = (T)0 + (dc[t] * v) * oc;
-                });
-            } else {
-                tail_spmv<T>(sm, R, c, [&](int t, T s) { bc[t] = mask[t] ? (T)0 : s; });
-            }
-            // a local level l - 1 is read next by CTA 0 alone; the other CTAs
-            // keep their r rows (read here remotely) until the next cluster
-            // barrier, which comes before any of them writes level l again
-            phase_end(Cl.local != 0);
-        }
-    }
-    {   // coarsest level: x0 = Ainv * b0 in FP64, one warp per own row (the order of k_coarse_gemv)
+    };
+    // coarsest level: x0 = Ainv * b0 in FP64, one warp per own row (the order of k_coarse_gemv)
+    auto coarse = [&]() {
         const TailLevel<T>& L0 = P.lv[0];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         const uint32_t bb = smem_u32(sm + L0.off_b);
@@ -365,41 +345,94 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
             if (lane == 0) x0[t] = (T)s;
         }
         phase_end(L0.local != 0 && (P.top < 1 || P.lv[1].local != 0));
+    };
+    if constexpr (FMG) {
+        phase_end(P.lv[P.top].local != 0);
+        for (int l = P.top; l >= 1; l--) {
+            const TailLevel<T>& Cl = P.lv[l - 1];
+            TailMat R = P.lv[l].R;
+            R.xoff = P.lv[l].off_b;
+            T* f = vec(Cl.off_b);
+            const unsigned char* mask = sm + Cl.off_mask;
+            tail_spmv<T>(sm, R, c, [&](int t, T s) { f[t] = mask[t] ? (T)0 : s; });
+            phase_end(Cl.local != 0);
+        }
+        coarse();
+    } else {
+        __syncthreads();
     }
-    for (int l = 1; l <= P.top; l++) {
-        const TailLevel<T>& L = P.lv[l];
-        const T* b = vec(L.off_b);
-        const T* dinv = vec(L.off_dinv);
-        const T om = L.omega;
-        {   // x += mask ? 0 : P x_{l-1}
-            T* x = vec(L.off_x);
-            const unsigned char* mask = sm + L.off_mask;
-            TailMat Pm = L.P;
-            Pm.xoff = P.lv[l - 1].off_x;
-            tail_spmv<T>(sm, Pm, c, [&](int t, T s) { x[t] = x[t] + (mask[t] ? (T)0 : s); });
-            phase_end(L.local != 0);
+    for (int lt = FMG ? 1 : P.top; lt <= P.top; lt++) {
+        for (int l = lt; l >= 1; l--) {
+            const TailLevel<T>& L = P.lv[l];
+            const bool loc = L.local != 0;
+            const bool entry = l == lt;
+            const T* b = vec(L.off_b);
+            if (FMG && entry) {   // x = P x_{l-1} as it is (no boundary zeroing), then all the sweeps
+                T* x = vec(L.off_x);
+                TailMat Pm = L.P;
+                Pm.xoff = P.lv[l - 1].off_x;
+                tail_spmv<T>(sm, Pm, c, [&](int t, T s) { x[t] = s; });
+                phase_end(loc);
+                sweeps(L, 0, L.off_x, loc);
+            } else {
+                // the first sweep from the zero guess lands where the last one ends in x
+                const int cur_off = (L.runs % 2 == 1) ? L.off_x : L.off_t;
+                if (entry) {   // below the entry level the restriction phase did it
+                    T* cur = vec(cur_off);
+                    const T* dinv = vec(L.off_dinv);
+                    const T om = L.omega;
+                    tail_own(L.Rl, L.n, c, [&](int t) { cur[t] = (T)0 + (dinv[t] * b[t]) * om; });
+                    phase_end(loc);
+                }
+                sweeps(L, 1, cur_off, loc);
+            }
+            {   // residual r = b - A x
+                T* r = vec(L.off_r);
+                TailMat A = L.A;
+                A.xoff = L.off_x;
+                tail_spmv<T>(sm, A, c, [&](int t, T s) { r[t] = b[t] - s; });
+                phase_end(loc);   // level l - 1 is local whenever level l is
+            }
+            {   // restriction into level l - 1 with zero boundary values (and its fused first sweep)
+                const TailLevel<T>& Cl = P.lv[l - 1];
+                TailMat R = L.R;
+                R.xoff = L.off_r;
+                T* bc = vec(Cl.off_b);
+                const unsigned char* mask = sm + Cl.off_mask;
+                if (l - 1 >= 1) {
+                    const T* dc = vec(Cl.off_dinv);
+                    T* xd = vec((Cl.runs % 2 == 1) ? Cl.off_x : Cl.off_t);
+                    const T oc = Cl.omega;
+                    tail_spmv<T>(sm, R, c, [&](int t, T s) {
+                        const T v = mask[t] ? (T)0 : s;
+                        bc[t] = v;
+                        xd[t] = (T)0 + (dc[t] * v) * oc;
+                    });
+                } else {
+                    tail_spmv<T>(sm, R, c, [&](int t, T s) { bc[t] = mask[t] ? (T)0 : s; });
+                }
+                // a local level l - 1 is read next by CTA 0 alone; the other CTAs
+                // keep their r rows (read here remotely) until the next cluster
+                // barrier, which comes before any of them writes level l again
+                phase_end(Cl.local != 0);
+            }
         }
-        // the last phase of level l is read next by the prolongation into
-        // level l + 1 (or, at the top, by the copy-out of the own rows)
-        const bool loc_next = L.local != 0 && (l == P.top || P.lv[l + 1].local != 0);
-        int cur_off = L.off_x;
-        for (int k = 0; k < L.runs; k++) {
-            const int alt_off = cur_off == L.off_x ? L.off_t : L.off_x;
-            const T* cu = vec(cur_off);
-            T* alt = vec(alt_off);
-            TailMat A = L.A;
-            A.xoff = cur_off;
-            tail_spmv<T>(sm, A, c, [&](int t, T s) { alt[t] = cu[t] + (dinv[t] * (b[t] - s)) * om; });
-            const bool last = k == L.runs - 1 && alt_off == L.off_x;
-            phase_end(last ? loc_next : L.local != 0);
-            cur_off = alt_off;
+        coarse();
+        for (int l = 1; l <= lt; l++) {
+            const TailLevel<T>& L = P.lv[l];
+            {   // x += mask ? 0 : P x_{l-1}
+                T* x = vec(L.off_x);
+                const unsigned char* mask = sm + L.off_mask;
+                TailMat Pm = L.P;
+                Pm.xoff = P.lv[l - 1].off_x;
+                tail_spmv<T>(sm, Pm, c, [&](int t, T s) { x[t] = x[t] + (mask[t] ? (T)0 : s); });
+                phase_end(L.local != 0);
+            }
+            // the last phase of level l is read next by the prolongation into
+            // level l + 1 (or, at the top, by the copy-out of the own rows)
+            sweeps(L, 0, L.off_x, L.local != 0 && (l == P.top || P.lv[l + 1].local != 0));
         }
-        if (cur_off != L.off_x) {
-            const T* cu = vec(cur_off);
-            T* x = vec(L.off_x);
-            tail_own(L.Rl, L.n, c, [&](int t) { x[t] = cu[t]; });
-            phase_end(loc_next);
-        }
+        if constexpr (!FMG) break;
     }
     {   // the result of the top level back to global memory
         const TailLevel<T>& L = P.lv[P.top];
@@ -408,7 +441,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
     }
 }
 
-template <typename T>
+template <typename T, bool FMG>
 void launch_tail(const TailParams<T>& p, int ctas, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};
@@ -429,18 +462,18 @@ void launch_tail(const TailParams<T>& p, int ctas, cudaStream_t st)
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    JFG_CUDA(cudaLaunchKernelEx(&cfg, k_mg_tail<T>, p));
+    JFG_CUDA(cudaLaunchKernelEx(&cfg, k_mg_tail<T, FMG>, p));
     note_launch();
 }
 
 // Largest cluster (16, else 8 CTAs) that can be resident with `smem` bytes
 // of dynamic shared memory per CTA; 0 when none can.
-template <typename T>
+template <typename T, bool FMG>
 int tail_cluster_size(size_t smem)
 {
     // the same cap for every hierarchy (the attribute belongs to the kernel, not to one launch)
-    JFG_CUDA(cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBudget));
-    JFG_CUDA(cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    JFG_CUDA(cudaFuncSetAttribute(k_mg_tail<T, FMG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBudget));
+    JFG_CUDA(cudaFuncSetAttribute(k_mg_tail<T, FMG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     for (int ctas : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ctas);
@@ -454,7 +487,7 @@ int tail_cluster_size(size_t smem)
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, k_mg_tail<T>, &cfg) == cudaSuccess && nc >= 1) return ctas;
+        if (cudaOccupancyMaxActiveClusters(&nc, k_mg_tail<T, FMG>, &cfg) == cudaSuccess && nc >= 1) return ctas;
         cudaGetLastError();
     }
     return 0;
@@ -641,6 +674,7 @@ template <typename T>
 void MGImpl<T>::build_tail()
 {
     tail = -1;
+    tail_full = false;
     const char* e = getenv("JFEM_MG_TAIL");
     if (e && e[0] == '0') return;
     cudaStream_t st = c->stream;
@@ -707,7 +741,7 @@ void MGImpl<T>::build_tail()
             if ((n[top] + cs - 1) / cs > kTailMaxRowsPerCta) continue;
             sizes(top, cs, pkg_b, tot_b);
             if (tot_b > (size_t)kTailSmemBudget) continue;
-            if (tail_cluster_size<T>(tot_b) >= cs) {
+            if (tail_cluster_size<T, false>(tot_b) >= cs) {
                 C = cs;
                 break;
             }
@@ -722,7 +756,7 @@ void MGImpl<T>::build_tail()
                 if (n[l] > kTailLocalRows) continue;
                 loc_rows = n[l];
                 sizes(top, C, pkg_b, tot_b);
-                if (tot_b <= (size_t)kTailSmemBudget && tail_cluster_size<T>(tot_b) >= C) break;
+                if (tot_b <= (size_t)kTailSmemBudget && tail_cluster_size<T, false>(tot_b) >= C) break;
                 loc_rows = 0;
             }
         }
@@ -811,6 +845,7 @@ void MGImpl<T>::build_tail()
     tail_smem_bytes = (int)tot_b;
     tail_ctas = C;
     tail = top;
+    tail_full = tail_cluster_size<T, true>(tot_b) >= C;
 }
 
 template <typename T>
@@ -938,14 +973,13 @@ void MGImpl<T>::smooth(int l, const T* rhs, bool xzero, const Scratch& sc, const
 }
 
 template <typename T>
-void MGImpl<T>::run_tail(bool first_sweep_done, const int* done, cudaStream_t st)
+void MGImpl<T>::run_tail(const T* rhs, bool full, const int* done, cudaStream_t st)
 {
-    (void)first_sweep_done;     // the tail redoes the top level's first sweep from b
     TailParams<T> p = {};
     p.top = tail;
     p.n0 = n[0];
     p.ainv0 = ainv0.p;
-    p.b_top = b[tail].p;
+    p.b_top = rhs;
     p.x_top = x[tail].p;
     p.done = done;
     p.pkg = tail_pkg.p;
@@ -969,7 +1003,10 @@ void MGImpl<T>::run_tail(bool first_sweep_done, const int* done, cudaStream_t st
         Lv.runs = sm[l].runs;
         Lv.omega = (T)sm[l].omega;
     }
-    launch_tail(p, tail_ctas, st);
+    if (full)
+        launch_tail<T, true>(p, tail_ctas, st);
+    else
+        launch_tail<T, false>(p, tail_ctas, st);
 }
 
 // mgStepV (MGPreconditionerInterface.java:125-198): guess in x[l] (or zero),
@@ -984,7 +1021,7 @@ void MGImpl<T>::vstep(int l, const T* rhs, bool xzero, const Scratch& sc, const 
         return;
     }
     if (l == tail && xzero && rhs == b[l].p) {   // the whole tail of the cycle in one cluster launch
-        run_tail(first_sweep_done, done, st);
+        run_tail(rhs, false, done, st);   // it redoes the top level's first sweep from rhs
         return;
     }
     if (l == 0) {
@@ -1036,12 +1073,17 @@ void MGImpl<T>::fmg_into_top(const T* defect, const Scratch& sc, const int* done
 {
     std::vector<const T*> rh(L);
     rh[L - 1] = defect;
-    for (int l = L - 2; l >= 0; l--) {
+    // the levels that the cluster holds run their part of the scheme in one launch
+    const int lo = tail_full ? tail : 0;
+    for (int l = L - 2; l >= lo; l--) {
         mg_spmv<T, 0>(*this, st, R[l], rh[l + 1], EpiMasked<T>{mask[l].p, fr[l].p}, sc, done);
         rh[l] = fr[l].p;
     }
-    for (int l = 0; l < L - 1; l++) {
-        vstep(l, rh[l], false, sc, done, st);
+    for (int l = lo; l < L - 1; l++) {
+        if (l == lo && lo > 0)
+            run_tail(rh[l], true, done, st);
+        else
+            vstep(l, rh[l], false, sc, done, st);
         // raw prolongation without boundary zeroing (getProlongationMatrix, line 323)
         mg_spmv<T, 0>(*this, st, P[l], x[l].p, EpiStore<T>{x[l + 1].p}, sc, done);
     }

@@ -36,6 +36,7 @@ struct MGImpl {
     int tail_ctas = 0;                      // CTAs of that cluster
     int tail_pkg_bytes = 0;                 // constant shared-memory package per CTA
     int tail_smem_bytes = 0;                // package + the level vectors per CTA
+    bool tail_full = false;                 // full multigrid on those levels as one launch too
     DevBuf<uint4> tail_pkg;                 // the matrices of levels 1..tail as per-CTA ELL slices
     std::vector<int> tail_meta;             // per level: shared-memory layout (see build_tail)
     std::vector<Matrix*> A, P, R;          // A[l], P[l] : n_{l+1} x n_l, R[l] = P[l]^T
@@ -91,7 +92,8 @@ struct MGImpl {
                 bool first_sweep_done = false, T* dest = nullptr);
     void coarse(const T* rhs, T* out, const int* done, cudaStream_t st);
     // the V-cycle below and including level `tail`, entered from the restriction above
-    void run_tail(bool first_sweep_done, const int* done, cudaStream_t st);
+    // (full: fullVCycleCorrection on the levels 0..tail); rhs of level tail, result in x[tail]
+    void run_tail(const T* rhs, bool full, const int* done, cudaStream_t st);
     void build_tail();
     void fmg_into_top(const T* defect, const Scratch& sc, const int* done, cudaStream_t st);
     int max_blocks() const;
