@@ -73,14 +73,6 @@ struct FinCGRes {    // after x += alpha p, r -= alpha Ap: t = ||r||^2
         check(c, sqrt(t[0]));
     }
 };
-struct FinBeta {     // beta = r'.z' / r.z
-    Ctl* c;
-    __device__ void operator()(const double* t) const
-    {
-        c->beta = t[0] / c->rz;
-        c->rz = t[0];
-    }
-};
 
 // ---------------------------------------------------------------------------
 // vector functors of the iterations
@@ -709,8 +701,17 @@ int run_cg(SolverWork& w, int ci, Matrix* A, const Precond<T>& M, const T* b, T*
         }
         vec_launch<1>(st, n, VCGUpdate<T>{x, p, r, Ap, c}, sc, done, FinCGRes{c, pcg ? 1 : 0});
         if (pcg) {
-            M.apply(r, z, sc, done, st);
-            vec_launch<1>(st, n, VDot<T>{r, z}, sc, done, FinBeta{c});
+            bool beta_done = false;
+            // r . z formed by the last sweep of an FP64 hierarchy; FP32 sweeps
+            // (and an FP32 hierarchy under FP64 iterates) keep the dot as a pass
+            // of its own: there the wider epilogue costs more than the launch
+            // (Q2 512 x 512 FP16: 2,612 us as a pass, 2,657 us fused; Q1 1024
+            // mixed 2,470 against 2,482; FP64 Q1 192: 564 against 550)
+            if (std::is_same<T, double>::value && M.kind == JFG_PREC_MG && !M.hook && !M.mg32)
+                beta_done = M.mg->apply(r, z, sc, done, st, c);
+            else
+                M.apply(r, z, sc, done, st);
+            if (!beta_done) vec_launch<1>(st, n, VDot<T>{r, z}, sc, done, FinBeta{c});
             vec_launch<0>(st, n, VXpby<T>{z, p, c}, sc, done);
         } else {
             vec_launch<0>(st, n, VXpby<T>{r, p, c}, sc, done);

@@ -68,26 +68,6 @@ __global__ void k_bc_defect(int naff, const int* __restrict__ row, const int* __
     d[r] = v[r] - s;
 }
 
-// k_bc_defect, and the first Jacobi sweep from zero of those rows:
-// y[r] = (dinv[r] * d[r]) * omega (the rest of y written by VCopyScaleMul)
-template <typename T>
-__global__ void k_bc_defect_scale(int naff, const int* __restrict__ row, const int* __restrict__ ptr,
-                                  const int* __restrict__ col, const T* __restrict__ val, const T* __restrict__ v,
-                                  T* __restrict__ d, const T* __restrict__ dinv, T* __restrict__ y, T omega,
-                                  const int* __restrict__ done)
-{
-    pdl_wait();
-    if (done && *done) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= naff) return;
-    int r = row[i];
-    T s = 0;
-    for (int k = ptr[i]; k < ptr[i + 1]; k++) s += val[k] * v[col[k]];
-    const T dr = v[r] - s;
-    d[r] = dr;
-    y[r] = (T)0 + (dinv[r] * dr) * omega;
-}
-
 // out[bd] += v[bd]   (initial.add(iterate), initial = boundary copy of v)
 template <typename T>
 __global__ void k_bc_add(int nb, const int* __restrict__ bd, const T* __restrict__ v, T* __restrict__ out,
@@ -270,8 +250,8 @@ __device__ __forceinline__ void tail_own(int R, int n, int c, F f)
 // lt only: those levels have had their turn, so no vector is added.
 // Bound, as the V-cycle's tail, by the latency of its phases (0.3 us on one
 // CTA, 0.7-1 us over the cluster); as launches each phase costs 3.5-5 us.
-// Q1 224 x 224, FP64, full multigrid and 3 V-cycles: 105 launches and 430 us
-// -> 36 launches and 345 us an application, the same sums in a row's order.
+// Q1 224 x 224, FP64, full multigrid and 3 V-cycles: 430 us in 105 launches
+// -> 345 us an application, the same sums in a row's order.
 template <typename T, bool FMG>
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_constant__ TailParams<T> P)
 {
@@ -612,11 +592,14 @@ void MGImpl<T>::init(Context* ctx, int levels, Matrix* const* As, Matrix* const*
         aff_ptr.alloc(naff + 1);
         aff_col.alloc(acol.size() ? acol.size() : 1);
         aff_val.alloc(aval.size() ? aval.size() : 1);
+        aff_mask.alloc(Af->rows);
+        if (Af->rows) JFG_CUDA(cudaMemsetAsync(aff_mask.p, 0, Af->rows, st));
         if (naff) {
             JFG_CUDA(cudaMemcpyAsync(aff_row.p, arow.data(), sizeof(int) * naff, cudaMemcpyHostToDevice, st));
             JFG_CUDA(cudaMemcpyAsync(aff_ptr.p, aptr.data(), sizeof(int) * (naff + 1), cudaMemcpyHostToDevice, st));
             JFG_CUDA(cudaMemcpyAsync(aff_col.p, acol.data(), sizeof(int) * acol.size(), cudaMemcpyHostToDevice, st));
             JFG_CUDA(cudaMemcpyAsync(aff_val.p, aval.data(), sizeof(T) * aval.size(), cudaMemcpyHostToDevice, st));
+            k_mask<<<nb(naff), 256, 0, st>>>(naff, aff_row.p, aff_mask.p);
         }
         JFG_CUDA(cudaStreamSynchronize(st));
     }
@@ -903,9 +886,13 @@ void MGImpl<T>::smooth(int l, const T* rhs, bool xzero, const Scratch& sc, const
         for (int k = 0; k < d.runs; k++) {
             T* o = (k == d.runs - 1) ? dest : alt;
             if (k == d.runs - 1 && bc_src && l == L - 1) {
-                mg_spmv<T, 0>(*this, st, M, cur, EpiJacobiBc<T>{cur, rhs, dinv[l].p, o, om, mask[l].p, bc_src}, sc,
-                              done);
+                const EpiJacobiBc<T> e{cur, rhs, dinv[l].p, o, om, mask[l].p, bc_src};
+                if (beta)
+                    mg_spmv<T, 1>(*this, st, M, cur, EpiJacobiBcDot<T>{e}, sc, done, FinBeta{beta});
+                else
+                    mg_spmv<T, 0>(*this, st, M, cur, e, sc, done);
                 bc_done = true;
+                beta_done = beta != nullptr;
             } else {
                 mg_spmv<T, 0>(*this, st, M, cur, EpiJacobi<T>{cur, rhs, dinv[l].p, o, om}, sc, done);
             }
@@ -1090,7 +1077,7 @@ void MGImpl<T>::fmg_into_top(const T* defect, const Scratch& sc, const int* done
 }
 
 template <typename T>
-void MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cudaStream_t st)
+bool MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cudaStream_t st, Ctl* ctl)
 {
     int Lf = L - 1, m = n[Lf];
     T* defect = b[Lf].p;
@@ -1101,11 +1088,10 @@ void MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cu
     if (fuse_first) {
         const T om = (T)sm[Lf].omega;
         T* dst0 = (sm[Lf].runs % 2 == 1) ? x[Lf].p : t[Lf].p;
-        vec_launch<0>(st, m, VCopyScaleMul<T>{v, defect, dinv[Lf].p, dst0, om}, sc, done);
-        if (naff)
-            launch_ex(k_bc_defect_scale<T>, dim3(nb(naff)), dim3(256), 0, st, naff, (const int*)aff_row.p,
-                      (const int*)aff_ptr.p, (const int*)aff_col.p, (const T*)aff_val.p, v, defect,
-                      (const T*)dinv[Lf].p, dst0, om, done);
+        vec_launch<0>(st, m + naff,
+                      VDefectScaleMul<T>{v, defect, dinv[Lf].p, dst0, om, m, aff_mask.p, aff_row.p, aff_ptr.p,
+                                         aff_col.p, aff_val.p},
+                      sc, done);
     } else {
         vec_launch<0>(st, m, VCopy<T>{v, defect}, sc, done);
         if (naff) {
@@ -1116,6 +1102,8 @@ void MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cu
     // the boundary add folded into the last post-smoothing sweep when it writes out
     bc_src = (nbd_fine && bd_unique) ? v : nullptr;
     bc_done = false;
+    beta = ctl;
+    beta_done = false;
     bool xzero = true;
     if (use_fmg && L > 1) {
         fmg_into_top(defect, sc, done, st);
@@ -1148,6 +1136,8 @@ void MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cu
     }
     bc_src = nullptr;
     bc_done = false;
+    beta = nullptr;
+    return beta_done;
 }
 
 template <typename T>

@@ -57,8 +57,11 @@ struct MGImpl {
     // (instead of a separate k_bc_add launch); bc_done reports that it did
     const T* bc_src = nullptr;
     bool bc_done = false;
+    Ctl* beta = nullptr;                    // apply()'s request, taken by that same sweep
+    bool beta_done = false;
     DevBuf<int> aff_row, aff_ptr, aff_col;
     DevBuf<T> aff_val;
+    DevBuf<unsigned char> aff_mask;         // 1 at the rows of aff_row
     int naff = 0;
     DevBuf<int> flags;                      // per-level smoother flags
     DevBuf<int> zero_flag;                  // a flag that stays 0
@@ -70,7 +73,9 @@ struct MGImpl {
 
     // out = M v (the preconditioner application).  v and out are device
     // vectors of the finest size; `done` is an optional skip flag.
-    void apply(const T* v, T* out, const Scratch& sc, const int* done, cudaStream_t st);
+    // With `ctl` the caller also wants v . out for the PCG's beta (FinBeta); the
+    // return value says whether that was done on the way.
+    bool apply(const T* v, T* out, const Scratch& sc, const int* done, cudaStream_t st, Ctl* ctl = nullptr);
     // out = vCycle(x0, rhs) on the finest level.
     void vcycle(const T* x0, const T* rhs, T* out, const Scratch& sc, const int* done, cudaStream_t st);
     // out = wCycle(x0, rhs) on the finest level.

@@ -106,6 +106,32 @@ struct EpiJacobiBc {  // EpiJacobi, then xn += v on the boundary rows (the MG mv
     }
 };
 
+struct FinBeta {     // beta = r'.z' / r.z
+    Ctl* c;
+    __device__ void operator()(const double* t) const
+    {
+        c->beta = t[0] / c->rz;
+        c->rz = t[0];
+    }
+};
+
+// EpiJacobiBc that also sums v . xn (the PCG's r . z: v is r, xn is z).  As a
+// pass of its own the dot is one more launch and reads both vectors again.
+// FP64 PCG, Q1 192 x 192: 564 -> 550 us; Q1 1024 x 1024: 3,096 -> 3,073 us.
+template <typename T>
+struct EpiJacobiBcDot {
+    EpiJacobiBc<T> e;
+    template <typename AT, int K>
+    __device__ void operator()(int r, AT s, double (&acc)[K]) const
+    {
+        const T vr = e.v[r];
+        T o = e.x[r] + (e.dinv[r] * (e.b[r] - (T)s)) * e.omega;
+        if (e.mask[r]) o = vr + o;
+        e.xn[r] = o;
+        acc[0] += (double)vr * (double)o;
+    }
+};
+
 template <typename T>
 struct EpiMasked {  // y = mask ? 0 : A x  (transfer followed by zero boundary values)
     const unsigned char* mask;
@@ -299,17 +325,37 @@ struct VScaleMul {  // y = (dinv * b) * omega      (first Jacobi sweep from a ze
     template <int K> __device__ void operator()(int i, double (&)[K]) const { y[i] = (T)0 + (dinv[i] * b[i]) * omega; }
 };
 template <typename T>
-struct VCopyScaleMul {  // d = v and y = (dinv * v) * omega: the defect copy fused with the first sweep from zero
+struct VDefectScaleMul {
+    // The defect d = v - A (v on the boundary) fused with the first sweep from
+    // zero, y = (dinv * d) * omega.  Indexes 0..n-1 are the rows whose entries
+    // in boundary columns are all zero (d = v; the others are marked in aff),
+    // indexes n.. the marked rows, each with its entries.  One launch: the
+    // marked rows as a kernel of their own cost 0.5-1 us an application behind
+    // the programmatic launch (PCG mixed Q1 1024: 2,488 -> 2,469 us, 17 applications).
     const T* v;
     T* d;
     const T* dinv;
     T* y;
     T omega;
+    int n;
+    const unsigned char* aff;
+    const int *row, *ptr, *col;
+    const T* val;
     template <int K> __device__ void operator()(int i, double (&)[K]) const
     {
-        const T vi = v[i];
-        d[i] = vi;
-        y[i] = (T)0 + (dinv[i] * vi) * omega;
+        int r = i;
+        T di;
+        if (i < n) {
+            di = v[i];
+            if (aff[i]) return;
+        } else {
+            r = row[i - n];
+            T s = 0;
+            for (int k = ptr[i - n]; k < ptr[i - n + 1]; k++) s += val[k] * v[col[k]];
+            di = v[r] - s;
+        }
+        d[r] = di;
+        y[r] = (T)0 + (dinv[r] * di) * omega;
     }
 };
 template <typename A, typename B>
