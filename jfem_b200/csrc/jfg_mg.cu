@@ -554,10 +554,18 @@ void MGImpl<T>::init(Context* ctx, int levels, Matrix* const* As, Matrix* const*
     }
     // finest boundary list and the rows with entries in boundary columns
     int Lf = L - 1;
-    nbd_fine = nbdry[Lf];
+    // (an unknown that the list names twice is one boundary unknown: its value is
+    // added once, and k_bc_add's threads write distinct rows)
+    std::vector<char> isbd(n[Lf], 0);
+    std::vector<int> bdl;
+    for (int i = 0; i < nbdry[Lf]; i++) {
+        if (!isbd[bdry[Lf][i]]) bdl.push_back(bdry[Lf][i]);
+        isbd[bdry[Lf][i]] = 1;
+    }
+    nbd_fine = (int)bdl.size();
     bd_fine.alloc(nbd_fine ? nbd_fine : 1);
     if (nbd_fine)
-        JFG_CUDA(cudaMemcpyAsync(bd_fine.p, bdry[Lf], sizeof(int) * nbd_fine, cudaMemcpyHostToDevice, st));
+        JFG_CUDA(cudaMemcpyAsync(bd_fine.p, bdl.data(), sizeof(int) * nbd_fine, cudaMemcpyHostToDevice, st));
     {
         Matrix* Af = A[Lf];
         std::vector<int> hp(Af->rows + 1);
@@ -567,11 +575,6 @@ void MGImpl<T>::init(Context* ctx, int levels, Matrix* const* As, Matrix* const*
         JFG_CUDA(cudaMemcpyAsync(hc.data(), Af->csr_col.p, sizeof(int) * Af->nnz, cudaMemcpyDeviceToHost, st));
         JFG_CUDA(cudaMemcpyAsync(hv.data(), Af->csr_val.p, sizeof(double) * Af->nnz, cudaMemcpyDeviceToHost, st));
         JFG_CUDA(cudaStreamSynchronize(st));
-        std::vector<char> isbd(Af->rows, 0);
-        for (int i = 0; i < nbd_fine; i++) {
-            if (isbd[bdry[Lf][i]]) bd_unique = false;
-            isbd[bdry[Lf][i]] = 1;
-        }
         std::vector<int> arow, aptr{0}, acol;
         std::vector<T> aval;
         for (int rr = 0; rr < Af->rows; rr++) {
@@ -1100,7 +1103,7 @@ bool MGImpl<T>::apply(const T* v, T* out, const Scratch& sc, const int* done, cu
         }
     }
     // the boundary add folded into the last post-smoothing sweep when it writes out
-    bc_src = (nbd_fine && bd_unique) ? v : nullptr;
+    bc_src = nbd_fine ? v : nullptr;
     bc_done = false;
     beta = ctl;
     beta_done = false;

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
     (1, 5, 4, 3, 2, "once"),      # only the last of two cycles forms the dot
     (2, 3, 4, 2, 1, "once"),      # SELL-32 rows
     (1, 5, 4, 2, 1, "none"),      # no boundary list on the finest level: the dot stays a pass of its own
-    (1, 5, 4, 2, 1, "twice"),     # an unknown named twice: the same
+    (1, 5, 4, 2, 1, "twice"),     # an unknown named twice counts once
 ])
 def test_pcg_matches_numpy(ctx, p, coarse, L, runs, cycles, boundary):
     """Residual history and solution against the PCG in NumPy with
