@@ -251,7 +251,7 @@ __device__ __forceinline__ void tail_own(int R, int n, int c, F f)
 // Bound, as the V-cycle's tail, by the latency of its phases (0.3 us on one
 // CTA, 0.7-1 us over the cluster); as launches each phase costs 3.5-5 us.
 // Q1 224 x 224, FP64, full multigrid and 3 V-cycles: 430 us in 105 launches
-// -> 345 us an application, the same sums in a row's order.
+// -> 345 us in 29 an application, the same sums in a row's order.
 template <typename T, bool FMG>
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_constant__ TailParams<T> P)
 {
