@@ -580,6 +580,9 @@ __global__ void __launch_bounds__(NT, NT > 512 ? 1 : 1024 / NT) k_batch_onchip(c
     const int nrow = cnt > tid ? (cnt - 1 - tid) / NT + 1 : 0;     // rows of this thread
     // every row of the warp regular (or absent): the passes run without a branch
     const bool plain = __all_sync(0xffffffffu, regular == (1u << nrow) - 1u);
+    // the halo in front too: a lower neighbour that owns fewer than H rows fills it in
+    // part only, and the absent rows' products read all of it (0 * what a kernel before left)
+    for (int t = tid; t < H; t += NT) zs[t] = 0.f;
     for (int t = cnt + H + tid; t < NT * RPT + 2 * H; t += NT) zs[t] = 0.f;   // read by absent rows: finite
     const float* zc = zs + H + tid;
     const float* z3[3] = {zc - str, zc, zc + str};
@@ -986,6 +989,14 @@ void plan_onchip(jfg_batch* b)
                 more = true;
             }
         }
+    }
+    // R is rounded up to whole warps, so the last CTAs of a wide cluster may own no
+    // row: they are left out (the same R, so the same rows and the same sums; 32 x 32
+    // cells at C = 16: R = 96, 12 CTAs)
+    for (int s = 0; s < b->nsys; s++) {
+        if (!b->oc_cluster[s]) continue;
+        const int need = (b->K[s]->rows + fits[s].R - 1) / fits[s].R;
+        if (need < b->oc_cluster[s] && resident[need]) b->oc_cluster[s] = need;
     }
     // launches: the largest clusters first (they need a whole GPC's free SMs),
     // within one the largest systems first
