@@ -545,7 +545,9 @@ void SolverWork::ensure(int n, int max_blocks, int hist_cap)
     partials.alloc(need);
     if (!counter.p) {
         counter.alloc(4);
-        JFG_CUDA(cudaMemset(counter.p, 0, 4 * sizeof(unsigned)));
+        // on the stream of the kernels that use it: the block may hold what its last
+        // owner left, and the legacy stream is not ordered with a non-blocking one
+        JFG_CUDA(cudaMemsetAsync(counter.p, 0, 4 * sizeof(unsigned), c->stream));
     }
     sc.partials = partials.p;
     sc.counter = counter.p;
