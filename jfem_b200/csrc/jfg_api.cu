@@ -122,6 +122,7 @@ int jfg_create(int device, jfg_ctx** out)
     ctx->c.device = device;
     int st = guard(ctx, [&]() -> int {
         JFG_CUDA(cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking));
+        jfg::pool_add_stream(device, ctx->c.stream);
         ctx->work.c = &ctx->c;
         return JFG_OK;
     });
@@ -141,6 +142,7 @@ int jfg_destroy(jfg_ctx* ctx)
     cudaStream_t s = ctx->c.stream;
     const int dev = ctx->c.device;
     delete ctx;
+    jfg::pool_drop_stream(dev, s);
     if (s) cudaStreamDestroy(s);
     jfg::pool_trim(dev);
     return JFG_OK;

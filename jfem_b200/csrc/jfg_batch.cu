@@ -751,6 +751,7 @@ struct jfg_batch {
         size_t smem = 0;
         cudaStream_t st = nullptr;
         cudaEvent_t done = nullptr;
+        int dev = 0;
     };
     std::vector<int> oc_cluster;
     std::vector<OnchipSys> oc_host;
@@ -763,7 +764,10 @@ struct jfg_batch {
     {
         for (auto& l : oc) {
             if (l.done) cudaEventDestroy(l.done);
-            if (l.st) cudaStreamDestroy(l.st);
+            if (!l.st) continue;
+            cudaStreamSynchronize(l.st);          // a call that failed half-way has not joined it
+            jfg::pool_drop_stream(l.dev, l.st);
+            cudaStreamDestroy(l.st);
         }
         if (oc_fork) cudaEventDestroy(oc_fork);
     }
@@ -1044,6 +1048,8 @@ void plan_onchip(jfg_batch* b)
         JFG_CUDA(cudaEventCreateWithFlags(&b->oc_fork, cudaEventDisableTiming));
         for (auto& l : b->oc) {
             JFG_CUDA(cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking));
+            l.dev = jfg::ctx_device(b->ctx);
+            jfg::pool_add_stream(l.dev, l.st);
             JFG_CUDA(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
         }
     }

@@ -47,6 +47,17 @@ struct Error {
 void* pool_alloc(size_t bytes, int* dev);
 void pool_free(void* p, size_t bytes, int dev) noexcept;
 void pool_trim(int dev) noexcept;
+// Every stream that the library launches on is made known to the pool before its
+// first use and taken off the list before it is destroyed.
+void pool_add_stream(int dev, cudaStream_t st);
+void pool_drop_stream(int dev, cudaStream_t st) noexcept;
+// Around each stream capture: no release waits for a stream meanwhile.
+struct CaptureScope {
+    CaptureScope();
+    ~CaptureScope();
+    CaptureScope(const CaptureScope&) = delete;
+    CaptureScope& operator=(const CaptureScope&) = delete;
+};
 
 template <typename T>
 struct DevBuf {

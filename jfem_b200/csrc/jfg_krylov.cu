@@ -582,6 +582,7 @@ int run_loop(SolverWork& w, const int* flag, const std::vector<uintptr_t>& key, 
                     cudaGraphNode_t node;
                     if (cudaGraphAddNode(&node, g, nullptr, 0, &p) == cudaSuccess) {
                         cudaGraph_t body = p.conditional.phGraph_out[0];
+                        CaptureScope capture;
                         JFG_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                                                cudaStreamCaptureModeThreadLocal));
                         unsigned long long before = g_launches.load();

@@ -4,13 +4,19 @@
 // cudaMalloc and again in cudaFree: 5.8 of the 9 ms of a Galerkin product of a
 // 263 k-row matrix.  A released block is kept, by device and size class, and
 // handed to the next allocation of that class.
-//   * Safety: a release waits for the device before the block may be handed out
-//     (cudaFree does the same), so no queued work of any stream still uses it;
-//     the lists are behind one mutex.
+//   * Safety: a block may be handed out once no queued work uses it any more.  All
+//     work of the library runs on the streams it has made (one per context, and
+//     those of the batched launches), so a release waits for these.  It does not
+//     wait for the device: that is an error, and breaks the capture, while any
+//     stream of the device is being captured, whoever's it is.  While a solver of
+//     this process captures (CaptureScope), or one of these streams is found
+//     capturing, the release is a plain cudaFree, which other threads may call
+//     during a thread-local capture.
 //   * Bound: at most kPoolCap bytes per device are kept, in blocks of at most
 //     kPoolBlock; what does not fit is freed at once.  pool_trim gives everything
 //     back (jfg_release_scratch, jfg_destroy, and before an allocation that the
 //     device refuses is tried again).
+#include <algorithm>
 #include <map>
 #include <mutex>
 
@@ -31,6 +37,34 @@ Pool& pool()
 {
     static Pool* p = new Pool();      // never destroyed: buffers of static objects outlive it otherwise
     return *p;
+}
+
+struct Streams {
+    std::mutex m;                                  // held while streams are waited for: no capture begins then
+    int capturing = 0;
+    std::map<int, std::vector<cudaStream_t>> of;   // the library's streams by device
+};
+Streams& streams()
+{
+    static Streams* s = new Streams();
+    return *s;
+}
+
+// Waits for the library's streams of a device; false when it may not or cannot.
+bool wait_streams(int dev)
+{
+    Streams& S = streams();
+    std::lock_guard<std::mutex> g(S.m);
+    if (S.capturing) return false;
+    for (cudaStream_t st : S.of[dev]) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            cudaGetLastError();                    // not the caller's: its next launch check may not find it
+            return false;
+        }
+    }
+    return true;
 }
 
 // eight classes per power of two, multiples of 512 bytes
@@ -89,18 +123,49 @@ void pool_free(void* b, size_t bytes, int dev) noexcept
     const size_t c = size_class(bytes);
     DeviceGuard on(dev);
     Pool& p = pool();
-    if (c <= kPoolBlock && cudaDeviceSynchronize() == cudaSuccess) {
+    if (c <= kPoolBlock) {
         try {
-            std::lock_guard<std::mutex> g(p.m);
-            if (p.kept[dev] + c <= kPoolCap) {
-                p.blocks[{dev, c}].push_back(b);
-                p.kept[dev] += c;
-                return;
+            if (wait_streams(dev)) {
+                std::lock_guard<std::mutex> g(p.m);
+                if (p.kept[dev] + c <= kPoolCap) {
+                    p.blocks[{dev, c}].push_back(b);
+                    p.kept[dev] += c;
+                    return;
+                }
             }
         } catch (...) {
         }
     }
     cudaFree(b);
+}
+
+void pool_add_stream(int dev, cudaStream_t st)
+{
+    Streams& S = streams();
+    std::lock_guard<std::mutex> g(S.m);
+    S.of[dev].push_back(st);
+}
+
+void pool_drop_stream(int dev, cudaStream_t st) noexcept
+{
+    Streams& S = streams();
+    std::lock_guard<std::mutex> g(S.m);
+    auto it = S.of.find(dev);
+    if (it == S.of.end()) return;
+    auto& v = it->second;
+    v.erase(std::remove(v.begin(), v.end(), st), v.end());
+}
+
+CaptureScope::CaptureScope()
+{
+    std::lock_guard<std::mutex> g(streams().m);
+    streams().capturing++;
+}
+
+CaptureScope::~CaptureScope()
+{
+    std::lock_guard<std::mutex> g(streams().m);
+    streams().capturing--;
 }
 
 void pool_trim(int dev) noexcept

@@ -27,3 +27,9 @@ def test_no_operation_on_the_legacy_stream():
             if commas < 3:
                 bad.append((f, m.group(0)))
     assert not bad, bad
+
+
+def test_no_wait_for_the_whole_device():
+    """cudaDeviceSynchronize is an error, and breaks the capture, while any stream of
+    the device is being captured by anyone in the process."""
+    assert [f for f, text in sources() if "cudaDeviceSynchronize" in text] == []
