@@ -67,11 +67,12 @@ bool wait_streams(int dev)
     return true;
 }
 
-// eight classes per power of two, multiples of 512 bytes
+// Eight classes per power of two, multiples of 512 bytes, up to steps of 2 MB (the
+// granularity of cudaMalloc, so a large block is no larger than it would be there).
 size_t size_class(size_t bytes)
 {
     size_t step = 512;
-    while (step * 16 <= bytes) step *= 2;
+    while (step * 16 <= bytes && step < ((size_t)2 << 20)) step *= 2;
     return (bytes + step - 1) / step * step;
 }
 
@@ -104,12 +105,13 @@ void* pool_alloc(size_t bytes, int* dev)
             return b;
         }
     }
+    const size_t size = c <= kPoolBlock ? c : bytes;      // a block that is never kept is not rounded up
     void* b = nullptr;
-    cudaError_t e = cudaMalloc(&b, c);
+    cudaError_t e = cudaMalloc(&b, size);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         pool_trim(*dev);
-        e = cudaMalloc(&b, c);
+        e = cudaMalloc(&b, size);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
