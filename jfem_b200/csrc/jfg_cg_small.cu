@@ -422,13 +422,8 @@ void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
     const char* e = getenv("JFEM_SMALL_CG_SMEM");
     const bool smem_ok = !(e && e[0] == '0') && R <= kSmMaxRows && bytes <= kSmemCap;
     if (smem_ok) {
-        static int attr_dev = -1;     // the opt-in shared memory size, set once per device
-        int dev = 0;
-        JFG_CUDA(cudaGetDevice(&dev));
-        if (attr_dev != dev) {
-            JFG_CUDA(cudaFuncSetAttribute(k_cg_small_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
-            attr_dev = dev;
-        }
+        static PerDevice once;
+        allow_smem(once, k_cg_small_smem, kSmemCap);
         k_cg_small_smem<<<kCgCtas, kSmThreads, bytes, st>>>(a, win, R, max_nnz, max_win);
     } else {
         k_cg_small<<<kCgCtas, kCgThreads, 0, st>>>(a);

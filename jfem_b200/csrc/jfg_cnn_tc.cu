@@ -818,11 +818,8 @@ static void launch_conv(cudaStream_t st, int B, int H, int W, const bf16* in, co
     if (grid <= 0) return;
     const CUtensorMap map = ws ? conv_input_map(B, H, W, in, 32, kRX, kBoxRows) : conv_input_map(B, H, W, in, 8, kHW, kHH);
     if (ws) {
-        static bool attr = false;
-        if (!attr) {
-            JFG_CUDA(cudaFuncSetAttribute(k_conv_ws<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem));
-            attr = true;
-        }
+        static PerDevice once;
+        allow_smem(once, k_conv_ws<MODE>, kDxSmem);
         k_conv_ws<MODE><<<grid, kDxThreads, kDxSmem, st>>>(map, B, H, W, w, aux, mask, out, out16, err, proj);
     } else if constexpr (MODE != kFwdProj) {
         k_conv_mid_tc<MODE><<<grid, kTcThreads, 0, st>>>(map, B, H, W, w, aux, mask, out, out16, err);
@@ -882,11 +879,8 @@ int wgrad_mid_tc(cudaStream_t st, int B, int H, int W, const __nv_bfloat16* G16,
     JFG_CHECK(ntiles < (1LL << 31), JFG_ERR_UNSUPPORTED, "image too large for the tensor-core weight gradient");
     const int ctas = (int)std::min<long long>(std::min<long long>(ntiles, sm_count()), max_parts);
     if (ctas <= 0) return 0;
-    static bool attr = false;
-    if (!attr) {
-        JFG_CUDA(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
-        attr = true;
-    }
+    static PerDevice once;
+    allow_smem(once, k_wgrad_tc, kWgSmem);
     const CUtensorMap tg = conv_input_map(B, H, W, G16, 32, kGTW, kGTH + 2);
     const CUtensorMap tx = conv_input_map(B, H, W, X, 32, kGTW, kGTH);
     k_wgrad_tc<<<ctas, kWgThreads, kWgSmem, st>>>(tg, tx, B, H, W, part, err);

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/jfem_gpu.h"
+#include "jfg_per_device.h"
 
 namespace jfg {
 
@@ -42,6 +43,16 @@ struct Error {
     do {                                                                                   \
         if (!(cond)) throw ::jfg::Error{(code), (text)};                                   \
     } while (0)
+
+// Lets a kernel take up to `bytes` of dynamic shared memory on the current device.
+template <class K>
+void allow_smem(PerDevice& once, K kern, size_t bytes)
+{
+    once.get([&] {
+        JFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return 1;
+    });
+}
 
 // device blocks kept between owners (jfg_pool.cu)
 void* pool_alloc(size_t bytes, int* dev);

@@ -726,12 +726,8 @@ void lu_solve_launch(int n, const double* LU, const int* piv, double* B, int nrh
     const char* e = getenv("JFEM_LU_BLOCKED");
     const size_t smem = (size_t)n * sizeof(double);
     if (smem <= kSolveSmemMax && !(e && e[0] == '0')) {
-        static bool attr = false;
-        if (!attr) {
-            JFG_CUDA(cudaFuncSetAttribute(k_lu_solve_blk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)kSolveSmemMax));
-            attr = true;
-        }
+        static PerDevice once;
+        allow_smem(once, k_lu_solve_blk, kSolveSmemMax);
         k_lu_solve_blk<<<nrhs, 512, smem, st>>>(n, LU, piv, B, nrhs);
     } else {
         k_lu_solve<<<nrhs, nrhs == 1 ? 1024 : 256, 0, st>>>(n, LU, piv, B, nrhs);
@@ -765,7 +761,8 @@ struct ClusterLaunch {
     }
 };
 
-// Largest cluster (at most 16) of `kern` with this block that can be resident; 0: none.
+// Largest cluster (at most 16) of `kern` with this block that can be resident on the
+// current device, which is made ready for its launch; 0: none.
 template <class K>
 int resident_cluster(K kern, int threads, size_t smem)
 {
@@ -786,21 +783,18 @@ int resident_cluster(K kern, int threads, size_t smem)
 // Whether one right-hand side of n unknowns goes through k_lu_solve_cl, and its cluster.
 int solve_cluster(int n)
 {
-    static const int max_c = resident_cluster(k_lu_solve_cl, kScMaxWarps * 32, 0);
+    static PerDevice once;
+    const int max_c = once.get([] { return resident_cluster(k_lu_solve_cl, kScMaxWarps * 32, 0); });
     const int nblk = (n + 31) / 32;
     const int C = std::min(max_c, std::max(1, nblk / 2));
     return C >= 1 && nblk <= C * kScMaxWarps ? C : 0;
 }
 
 // Whether a 16-CTA cluster of k_lu_panel_cl with the largest dynamic shared
-// memory it is launched with (200 KB per CTA) can be resident; asked once per
-// process, on the first device that factors a large enough matrix.
-bool panel_cluster_ok()
+// memory it is launched with (200 KB per CTA) can be resident.
+bool panel_cluster_fits()
 {
-    static int cached = -1;
-    if (cached >= 0) return cached == 1;
     constexpr size_t kMax = 200 * 1024;
-    cached = 0;
     if (cudaFuncSetAttribute(k_lu_panel_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) != cudaSuccess ||
         cudaFuncSetAttribute(k_lu_panel_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
@@ -818,9 +812,14 @@ bool panel_cluster_ok()
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, k_lu_panel_cl, &cfg) == cudaSuccess && nc >= 1) cached = 1;
+    const bool ok = cudaOccupancyMaxActiveClusters(&nc, k_lu_panel_cl, &cfg) == cudaSuccess && nc >= 1;
     cudaGetLastError();
-    return cached == 1;
+    return ok;
+}
+bool panel_cluster_ok()
+{
+    static PerDevice once;
+    return once.get([] { return (int)panel_cluster_fits(); }) != 0;
 }
 
 void launch_panel(int n, double* A, int* piv, int k0, int nb, int* info, cudaStream_t st)
@@ -828,7 +827,8 @@ void launch_panel(int n, double* A, int* piv, int k0, int nb, int* info, cudaStr
     const int R = n - k0;
     const int rc = (R + kPcCtas - 1) / kPcCtas;
     const size_t smem = (size_t)rc * kPcStride * sizeof(double);
-    static const int max_reg = resident_cluster(k_lu_panel_reg, kPrThreads, kPrSmem);
+    static PerDevice once;
+    const int max_reg = once.get([] { return resident_cluster(k_lu_panel_reg, kPrThreads, kPrSmem); });
     const int C = (R + kPrThreads - 1) / kPrThreads;
     if (C <= max_reg) {
         ClusterLaunch l(C, kPrThreads, kPrSmem, st);

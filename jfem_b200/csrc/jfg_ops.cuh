@@ -201,11 +201,8 @@ void launch_pt_kind(cudaStream_t st, const Matrix* M, const VT* val, const XT* x
     const int smem = pt_smem<VT>(KIND == 1 ? 4 : 9);
     auto kern = k_spmv_pt<VT, XT, NR, Epi, Fin, PF, KIND>;
     if (smem > 48 * 1024) {
-        static const bool set = [&] {
-            JFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            return true;
-        }();
-        (void)set;
+        static PerDevice once;
+        allow_smem(once, kern, smem);
     }
     PtArgs a{M->st_S, M->st_S2, M->st_lo, nreg, M->st_ld, M->st_nirr, ntiles, M->st_irow.p, M->st_iptr.p,
              M->st_icol.p, std::is_same<VT, __half>::value ? M->hscale_inv : 1.0f, M->st_err.p};

@@ -1217,23 +1217,15 @@ void SchwarzImpl::colour_step(const Colour& col, const T* b, T* x, double om, co
                 k_schwarz_batch<T, IT, kBatchThreads><<<col.b_count, kBatchThreads, 0, st>>>(
                     csr_of(A), bpat.p, bptr.p + col.b_start, pptr.p, dofs.p, inv_off.p, iv, b, x, om, done);
         } else if (col.kern == 2) {
-            static bool attr = false;      // per instantiation
-            if (!attr) {
-                JFG_CUDA(cudaFuncSetAttribute(k_schwarz_colour<T, IT, true>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmemMax));
-                attr = true;
-            }
+            static PerDevice once;         // per instantiation
+            allow_smem(once, k_schwarz_colour<T, IT, true>, kColSmemMax);
             const size_t smem = col_smem_inv<IT>(col.mcap) + col_smem_rows(col.rows_cap);
             k_schwarz_colour<T, IT, true><<<col.grid, kColThreads, smem, st>>>(
                 csr_of(A), bpat.p, bptr.p + col.b_start, col.b_count, pptr.p, dofs.p, inv_off.p, iv, col.mcap,
                 col.rows_cap, b, x, om, done);
         } else if (col.kern == 3) {
-            static bool attr = false;      // per instantiation
-            if (!attr) {
-                JFG_CUDA(cudaFuncSetAttribute(k_schwarz_colour<T, IT, false>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmemMax));
-                attr = true;
-            }
+            static PerDevice once;         // per instantiation
+            allow_smem(once, k_schwarz_colour<T, IT, false>, kColSmemMax);
             k_schwarz_colour<T, IT, false><<<col.grid, kColThreads, col_smem_rows(col.rows_cap), st>>>(
                 csr_of(A), bpat.p, bptr.p + col.b_start, col.b_count, pptr.p, dofs.p, inv_off.p, iv, col.mcap,
                 col.rows_cap, b, x, om, done);
@@ -1272,14 +1264,11 @@ void SchwarzImpl::sweep(int runs, const T* b, T* x, const int* done, cudaStream_
     P.ncol = (int)colours.size();
     P.rounds = sweep_rounds;
     auto* kern = sweep_smem ? k_schwarz_sweep<T, IT, true> : k_schwarz_sweep<T, IT, false>;
-    static bool attr = false;          // per instantiation
-    if (!attr) {
-        JFG_CUDA(cudaFuncSetAttribute(k_schwarz_sweep<T, IT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kColSmemMax));
-        JFG_CUDA(cudaFuncSetAttribute(k_schwarz_sweep<T, IT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kColSmemMax));
-        attr = true;
-    }
+    static PerDevice with_smem, without;   // per instantiation
+    if (sweep_smem)
+        allow_smem(with_smem, k_schwarz_sweep<T, IT, true>, kColSmemMax);
+    else
+        allow_smem(without, k_schwarz_sweep<T, IT, false>, kColSmemMax);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)sweep_grid);
     cfg.blockDim = dim3(kSwThreads);
