@@ -4,11 +4,10 @@
 // entries in registers; the two dot products of an iteration are reduced through
 // distributed shared memory (every CTA sums the eight CTA partials in rank
 // order, so every thread holds the same value and takes the same branch).
-// Two cluster barriers per iteration with the matrix in shared memory
-// (k_cg_small_smem), three with p in global memory (k_cg_small), replace the ~5
-// kernel launches of the graph-captured loop, whose launch latency dominates at
-// this size.  The
-// scalar recurrences and the stopping test are those of the multi-kernel CG
+// Two or three cluster barriers per iteration with the matrix in shared memory
+// (k_cg_small_smem<true>, <false>), three with p in global memory (k_cg_small),
+// replace the ~5 kernel launches of the graph-captured loop, whose launch latency
+// dominates at this size.  The scalar recurrences and the stopping test are those of the multi-kernel CG
 // (alpha = rz / p.Ap, beta = rr' / rr, `iter < maxit && ||r|| > tol`,
 // NONFINITE on a non-finite residual); the loop is bounded by maxit.
 #include <cooperative_groups.h>
@@ -30,6 +29,7 @@ constexpr int kCgRowsPerThread = 2;
 constexpr int kSmThreads = 512;      // shared-memory variant: 512 threads x 4 rows
 constexpr int kSmRows = 4;
 constexpr int kSmMaxRows = 2048;     // rows per CTA of the shared-memory variant
+constexpr size_t kSmSmemCap = (size_t)200 * 1024;
 
 struct CgSmallArgs {
     int n;
@@ -191,7 +191,13 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads, 1)
 // sum is one push per CTA into a slot of every other, then eight local loads in
 // rank order.  Bound by those two rounds (~1,400 cycles each); with p itself
 // broadcast to all CTAs, a third barrier for it and sums read remotely, an
-// iteration at 4,225 rows took 5.2 us.  Used when slice and windows fit.
+// iteration at 4,225 rows took 5.2 us.
+// R_WINDOW = false keeps the window of p alone: the owners push p once beta is
+// known and a third barrier follows.  The same sums, the same bits, in half of the
+// windows' bytes: it takes numberings whose windows are too wide for both (random
+// orders, ~6,800 to ~9,300 rows at nine entries each).
+// 100 iterations at 8,464 rows in random order, the whole call: 779 us, against
+// 1,456 us in k_cg_small; in the grid's order, with both windows, 547 us.
 struct CgRange {
     int nnz, lo, hi;    // CSR slice and window of a CTA
 };
@@ -225,7 +231,10 @@ __global__ void __launch_bounds__(256) k_cg_small_range(int n, int R, const int*
     }
 }
 
-// cluster_sum with the partials pushed: the same sums in the same order; slot[kCgCtas] has one call site
+// cluster_sum with the partials pushed: the same sums in the same order.  Between two
+// uses of one slot[kCgCtas] lies a sum through another, or the start of the loop:
+// its readers are past it (slot_rr is used before the loop and at its end, slot_pap
+// between the two).
 __device__ __forceinline__ double pushed_sum(cg::cluster_group& cl, double v, double* warp_part, double* slot)
 {
     v = warp_sum(v);
@@ -245,6 +254,7 @@ __device__ __forceinline__ double pushed_sum(cg::cluster_group& cl, double v, do
     return t;
 }
 
+template <bool R_WINDOW>
 __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
     k_cg_small_smem(CgSmallArgs a, const __grid_constant__ CgWindows win, int R, int max_nnz, int max_win)
 {
@@ -252,8 +262,8 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
     __shared__ double warp_part[kSmThreads / 32];
     __shared__ double slot_pap[kCgCtas], slot_rr[kCgCtas];
     double* pw = reinterpret_cast<double*>(smem);                          // max_win
-    double* rw = pw + max_win;                                             // max_win
-    double* lval = rw + max_win;                                           // max_nnz
+    double* rw = pw + max_win;                                             // max_win (R_WINDOW)
+    double* lval = R_WINDOW ? rw + max_win : rw;                           // max_nnz
     int* lptr = reinterpret_cast<int*>(lval + max_nnz);                    // R + 1
     int* lcol = lptr + R + 1;                                              // max_nnz
     cg::cluster_group cl = cg::this_cluster();
@@ -303,14 +313,14 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
         }
         return s;
     };
-    auto push_r = [&]() {
+    auto push = [&](double* w, const double (&v)[kSmRows]) {  // the own rows' v into the windows w that hold them
 #pragma unroll
         for (int j = 0; j < kSmRows; j++)
             if (rows[j] < nr) {
                 const int g = r0 + rows[j];
 #pragma unroll
                 for (int t = 0; t < kCgCtas; t++)
-                    if (g >= win.c[t].lo && g < win.c[t].hi) *cl.map_shared_rank(rw + (g - win.c[t].lo), t) = r[j];
+                    if (g >= win.c[t].lo && g < win.c[t].hi) *cl.map_shared_rank(w + (g - win.c[t].lo), t) = v[j];
             }
     };
     // r = b - A x0, rr
@@ -321,7 +331,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
             r[j] = a.b[r0 + rows[j]] - local_dot(rows[j]);
             part += r[j] * r[j];
         }
-    push_r();
+    if constexpr (R_WINDOW) push(rw, r);
     double rr = pushed_sum(cl, part, warp_part, slot_rr);
     double rz = rr;
     int iter = 0, status = JFG_NOT_CONVERGED, not_pd = 0;
@@ -329,8 +339,13 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
     bool done = stop_test(c, res, iter, maxit, tol, &status);
 #pragma unroll
     for (int j = 0; j < kSmRows; j++) p[j] = r[j];
-    for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i];
-    __syncthreads();
+    if constexpr (R_WINDOW) {
+        for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i];
+        __syncthreads();
+    } else {
+        push(pw, p);                                          // x0 has been read: the sum's barrier
+        cl.sync();
+    }
     while (!done) {
         part = 0.0;
 #pragma unroll
@@ -350,7 +365,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
                 r[j] = r[j] - ap[j] * alpha;
                 part += r[j] * r[j];
             }
-        push_r();
+        if constexpr (R_WINDOW) push(rw, r);
         const double rr_new = pushed_sum(cl, part, warp_part, slot_rr);
         iter++;
         const double beta = rr_new / rr;
@@ -363,8 +378,13 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kSmThreads, 1)
 #pragma unroll
         for (int j = 0; j < kSmRows; j++)
             if (rows[j] < nr) p[j] = r[j] + p[j] * beta;
-        for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i] + pw[i] * beta;
-        __syncthreads();
+        if constexpr (R_WINDOW) {
+            for (int i = threadIdx.x; i < W; i += kSmThreads) pw[i] = rw[i] + pw[i] * beta;
+            __syncthreads();
+        } else {
+            push(pw, p);
+            cl.sync();
+        }
     }
 #pragma unroll
     for (int j = 0; j < kSmRows; j++)
@@ -389,6 +409,22 @@ bool cg_small_fits(const Matrix* A)
     return !(e && e[0] == '0') && A->rows <= kCgCtas * kCgThreads * kCgRowsPerThread;
 }
 
+static size_t cg_small_bytes(int n, int max_nnz, int max_win, int windows)
+{
+    const size_t R = (size_t)(n + kCgCtas - 1) / kCgCtas;
+    return sizeof(double) * ((size_t)windows * max_win + max_nnz) + sizeof(int) * (R + 1 + max_nnz) + 16;
+}
+
+// Windows that the shared-memory variant keeps beside the largest CSR slice of a
+// row block: of p and r (2), of p alone (1), or 0: k_cg_small.
+int cg_small_windows(int n, int max_nnz, int max_win)
+{
+    if ((n + kCgCtas - 1) / kCgCtas > kSmMaxRows) return 0;
+    for (int w : {2, 1})
+        if (cg_small_bytes(n, max_nnz, max_win, w) <= kSmSmemCap) return w;
+    return 0;
+}
+
 // Runs the whole CG; the control block w.ctl[0] holds tol / maxit / history
 // on entry and the results on return (as the multi-kernel loop leaves them).
 void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
@@ -397,7 +433,7 @@ void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
     const int n = A->rows;
     w.v64[0].alloc((size_t)n);
     CgSmallArgs a{n, A->csr_ptr.p, A->csr_col.p, A->csr_val.p, b, x, w.v64[0].p, w.ctl.p};
-    // shared-memory variant when a CTA's CSR slice and its windows of p and r fit
+    // shared-memory variant when a CTA's CSR slice and its windows of p and r, or of p, fit
     const int R = (n + kCgCtas - 1) / kCgCtas;
     if (A->cg_small_win.size() != kCgCtas * 3) {      // once per matrix: slices and windows of the row blocks
         DevBuf<CgRange> d;
@@ -417,14 +453,21 @@ void run_cg_small(SolverWork& w, Matrix* A, const double* b, double* x)
         max_nnz = std::max(max_nnz, win.c[q].nnz);
         max_win = std::max(max_win, win.c[q].hi - win.c[q].lo);
     }
-    const size_t bytes = sizeof(double) * (2 * (size_t)max_win + max_nnz) + sizeof(int) * ((size_t)R + 1 + max_nnz) + 16;
-    constexpr size_t kSmemCap = (size_t)200 * 1024;
+    // JFEM_SMALL_CG_SMEM: "0" keeps p in global memory, "p" the window of p alone
     const char* e = getenv("JFEM_SMALL_CG_SMEM");
-    const bool smem_ok = !(e && e[0] == '0') && R <= kSmMaxRows && bytes <= kSmemCap;
-    if (smem_ok) {
+    int windows = cg_small_windows(n, max_nnz, max_win);
+    if (e && e[0] == '0') windows = 0;
+    if (e && e[0] == 'p') windows = std::min(windows, 1);
+    if (windows) {
+        const size_t bytes = cg_small_bytes(n, max_nnz, max_win, windows);
         static PerDevice once;
-        allow_smem(once, k_cg_small_smem, kSmemCap);
-        k_cg_small_smem<<<kCgCtas, kSmThreads, bytes, st>>>(a, win, R, max_nnz, max_win);
+        once.get([] {
+            for (auto kern : {k_cg_small_smem<true>, k_cg_small_smem<false>})
+                JFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmSmemCap));
+            return 1;
+        });
+        auto* kern = windows == 2 ? k_cg_small_smem<true> : k_cg_small_smem<false>;
+        kern<<<kCgCtas, kSmThreads, bytes, st>>>(a, win, R, max_nnz, max_win);
     } else {
         k_cg_small<<<kCgCtas, kCgThreads, 0, st>>>(a);
     }
