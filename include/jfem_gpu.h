@@ -254,7 +254,10 @@ int jfg_schwarz_info(jfg_schwarz* s, int* max_patch, int64_t* inverse_entries, i
 int jfg_schwarz_apply(jfg_schwarz* s, const double* h_rhs, double* h_x);
 /* out = SubspaceCorrection.solve(schwarz, rhs) = AbstractSchwarz.mvMul (AbstractSchwarz.java:62-66). */
 int jfg_schwarz_solve(jfg_schwarz* s, const double* h_rhs, double* h_out);
-/* x <- SchwarzSmoother.smooth: runs x apply. */
+/* x <- SchwarzSmoother.smooth: runs x apply.  Coloured sweeps that run as one launch
+ * have bounded waits: a call in which one ran out (smoothing, a V-cycle or a solve
+ * that smooths) returns JFG_ERR_CUDA; of a call that does not wait for its work the
+ * next call on the context does.  The handle stays usable. */
 int jfg_schwarz_smooth(jfg_schwarz* s, int runs, const double* h_rhs, double* h_x);
 int jfg_schwarz_smooth_dev(jfg_schwarz* s, int runs, const double* d_rhs, double* d_x);
 /* Patch p's size, sorted DOFs and row-major inverse (each output may be NULL). */

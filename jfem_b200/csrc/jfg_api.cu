@@ -42,8 +42,10 @@ int guard(jfg_ctx* ctx, F&& f)
         if (ctx) {
             cudaError_t e = cudaSetDevice(ctx->c.device);
             if (e != cudaSuccess) throw Error{JFG_ERR_CUDA, cudaGetErrorString(e)};
+            ctx->c.check_sweeps();     // of a call that did not wait for its work
         }
         int st = f();
+        if (ctx) ctx->c.check_sweeps();
         if (ctx && st != JFG_OK && ctx->c.last_error.empty()) ctx->c.last_error = "status " + std::to_string(st);
         return st;
     } catch (const Error& e) {

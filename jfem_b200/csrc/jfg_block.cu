@@ -20,6 +20,7 @@ namespace jfg {
 cudaStream_t ctx_stream(jfg_ctx* ctx);
 int ctx_device(jfg_ctx* ctx);
 void ctx_set_error(jfg_ctx* ctx, const std::string& msg);
+Context* ctx_context(jfg_ctx* ctx);
 
 namespace {
 
@@ -118,6 +119,7 @@ int jfg_blockdiag_apply(jfg_blockdiag* b, const double* h_v, double* h_out)
         jfg::blockdiag_apply(b, v.p, z.p, sc, nullptr, st);
         JFG_CUDA(cudaMemcpyAsync(h_out, z.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
         JFG_CUDA(cudaStreamSynchronize(st));
+        jfg::ctx_context(b->ctx)->check_sweeps();
         return JFG_OK;
     } catch (const jfg::Error& e) {
         jfg::ctx_set_error(b->ctx, e.msg);

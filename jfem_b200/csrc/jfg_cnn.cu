@@ -685,6 +685,7 @@ namespace jfg {
 cudaStream_t ctx_stream(jfg_ctx* ctx);
 int ctx_device(jfg_ctx* ctx);
 void ctx_set_error(jfg_ctx* ctx, const std::string& msg);
+Context* ctx_context(jfg_ctx* ctx);
 }  // namespace jfg
 
 struct jfg_cnn {
@@ -1283,6 +1284,7 @@ int jfg_mgcnn_apply_dev(jfg_mgcnn* p, const double* d_v, double* d_z)
         jfg::Scratch sc{p->partials.p, p->counter.p};
         jfg::mgcnn_apply(p, d_v, d_z, sc, nullptr, st);
         JFG_CUDA(cudaStreamSynchronize(st));
+        jfg::ctx_context(p->ctx)->check_sweeps();
         return JFG_OK;
     } catch (const jfg::Error& e) {
         jfg::ctx_set_error(p->ctx, e.msg);

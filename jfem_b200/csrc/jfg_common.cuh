@@ -207,6 +207,22 @@ struct Context {
     DevBuf<double> scal;          // small scalar results
     // grow-only scratch of the sparse products (per-row counts; products and sort space)
     DevBuf<char> gemm_rows, gemm_ws;
+    // The coloured Schwarz sweeps (k_schwarz_sweep) report a grid barrier that ran
+    // out: a device word that ends the sweeps queued behind it at once, and a pinned
+    // word that the host reads without a copy.  Null until a sweep is planned.
+    DevBuf<unsigned> sweep_err;
+    volatile unsigned* sweep_fault = nullptr;
+    void plan_sweeps();
+    // Throws when a sweep of this context ran out, after clearing both words.
+    void check_sweeps()
+    {
+        if (sweep_fault && *sweep_fault) sweep_failed();
+    }
+    void sweep_failed();
+    Context() = default;
+    Context(const Context&) = delete;
+    Context& operator=(const Context&) = delete;
+    ~Context();
 };
 
 // host-side helpers implemented in jfg_matrix.cu

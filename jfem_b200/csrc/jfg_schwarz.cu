@@ -546,17 +546,21 @@ __global__ void __launch_bounds__(kColThreads, 1)
 // the same bits.
 //
 // The barrier is a counter in global memory that every CTA increments once per
-// step; the wait is bounded (about a second), after which the CTA sets the error
-// word, writes NaN into one of its x entries (the caller's iteration then reports
-// a non-finite value) and leaves; a set error word makes later launches do the
-// same at once.  The last CTA to leave re-arms the counters.
+// step; the wait is bounded (about a second; JFEM_SCHWARZ_SWEEP_SPINS sets the
+// polls), after which the CTA sets the context's error words, writes NaN into one of
+// its x entries (the caller's iteration then ends on a non-finite value) and leaves;
+// a set error word makes later launches do the same at once.  The last CTA to leave
+// re-arms the counters.  The call that finds the error returns it and clears the
+// words (Context::check_sweeps), so that the next sweep runs.
 // ---------------------------------------------------------------------------
 constexpr int kSwMaxColours = 16;
 constexpr int kSwPre = kRowUnroll;            // prefetched entries per lane (kRowLanes lanes per row)
 constexpr int kSwThreads = 672;               // 96 registers, 168 rows per pass; patches up to this size
 
 struct SweepParams {
-    int ncol, runs, rounds;
+    int ncol, runs, rounds, spins;
+    unsigned* err;                 // Context::sweep_err
+    volatile unsigned* fault;      // Context::sweep_fault
 };
 
 __global__ void k_sweep_rows(int nb, const int* __restrict__ bpat, const int* __restrict__ bptr,
@@ -598,7 +602,7 @@ __global__ void __launch_bounds__(kSwThreads, 1)
         else
             sbd[tid].np = 0;
     }
-    if (tid == 0) s_ok = *reinterpret_cast<volatile unsigned*>(bar + 2) == 0;
+    if (tid == 0) s_ok = *reinterpret_cast<volatile unsigned*>(P.err) == 0;
     __syncthreads();
     int64_t loaded = -1;                                           // the inverse in shared memory
     // state fetched ahead of the barrier: the residual row's entries, its right-hand side, DOF
@@ -713,7 +717,7 @@ __global__ void __launch_bounds__(kSwThreads, 1)
             const unsigned want = (unsigned)(s + 1) * (unsigned)G;
             bool in = false;
 #pragma unroll 1
-            for (int i = 0; i < (1 << 21) && !in; i++) {
+            for (int i = 0; i < P.spins && !in; i++) {
                 unsigned now;
                 asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
                 in = now >= want;
@@ -727,7 +731,9 @@ __global__ void __launch_bounds__(kSwThreads, 1)
     cp_async_wait<0>();
     if (tid == 0) {
         if (!ok) {
-            atomicOr(bar + 2, 1u);
+            atomicOr(P.err, 1u);
+            *P.fault = 1u;
+            __threadfence_system();
             x[brow[0].x] = (T)NAN;
         }
         __threadfence();
@@ -1171,8 +1177,9 @@ void SchwarzImpl::plan_sweep(const std::vector<int>& h_bpat, const std::vector<i
     JFG_CUDA(cudaMemcpyAsync(bslot.p, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice, st));
     bdesc.alloc(d.size());
     brow.alloc((size_t)row0);
-    bar.alloc(4);
-    JFG_CUDA(cudaMemsetAsync(bar.p, 0, 4 * sizeof(unsigned), st));
+    bar.alloc(2);
+    JFG_CUDA(cudaMemsetAsync(bar.p, 0, 2 * sizeof(unsigned), st));
+    this->c->plan_sweeps();
     JFG_CUDA(cudaMemcpyAsync(bdesc.p, d.data(), sizeof(BatchDesc) * d.size(), cudaMemcpyHostToDevice, st));
     k_sweep_rows<<<(unsigned)d.size(), 256, 0, st>>>((int)d.size(), bpat.p, bptr.p, bdesc.p, pptr.p, dofs.p,
                                                     A->csr_ptr.p, brow.p);
@@ -1180,6 +1187,30 @@ void SchwarzImpl::plan_sweep(const std::vector<int>& h_bpat, const std::vector<i
     note_launch();
     JFG_CUDA(cudaStreamSynchronize(st));
     sweep_grid = grid;
+}
+
+void Context::plan_sweeps()
+{
+    if (sweep_fault) return;
+    sweep_err.alloc(1);
+    JFG_CUDA(cudaMemsetAsync(sweep_err.p, 0, sizeof(unsigned), stream));
+    void* h = nullptr;
+    JFG_CUDA(cudaHostAlloc(&h, sizeof(unsigned), cudaHostAllocMapped));
+    sweep_fault = static_cast<volatile unsigned*>(h);
+    *sweep_fault = 0;
+}
+
+void Context::sweep_failed()
+{
+    cudaStreamSynchronize(stream);     // the sweeps queued behind it have left too
+    *sweep_fault = 0;
+    JFG_CUDA(cudaMemsetAsync(sweep_err.p, 0, sizeof(unsigned), stream));
+    throw Error{JFG_ERR_CUDA, "coloured Schwarz sweep: a wait for the other CTAs ran out"};
+}
+
+Context::~Context()
+{
+    if (sweep_fault) cudaFreeHost(const_cast<unsigned*>(sweep_fault));
 }
 
 const float* SchwarzImpl::inverses32()
@@ -1263,6 +1294,10 @@ void SchwarzImpl::sweep(int runs, const T* b, T* x, const int* done, cudaStream_
     P.runs = runs;
     P.ncol = (int)colours.size();
     P.rounds = sweep_rounds;
+    const char* e = getenv("JFEM_SCHWARZ_SWEEP_SPINS");
+    P.spins = e && *e ? atoi(e) : 1 << 21;
+    P.err = c->sweep_err.p;
+    P.fault = c->sweep_fault;
     auto* kern = sweep_smem ? k_schwarz_sweep<T, IT, true> : k_schwarz_sweep<T, IT, false>;
     static PerDevice with_smem, without;   // per instantiation
     if (sweep_smem)
@@ -1378,7 +1413,11 @@ int sguard(jfg_ctx* ctx, F&& f)
 {
     try {
         JFG_CUDA(cudaSetDevice(jfg::ctx_device(ctx)));
-        return f();
+        jfg::Context* c = jfg::ctx_context(ctx);
+        c->check_sweeps();             // of a call that did not wait for its work
+        const int st = f();
+        c->check_sweeps();
+        return st;
     } catch (const jfg::Error& e) {
         jfg::ctx_set_error(ctx, e.msg);
         return e.status;

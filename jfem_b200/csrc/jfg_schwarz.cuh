@@ -45,7 +45,7 @@ struct SchwarzImpl {
     };
     DevBuf<BatchDesc> bdesc;
     DevBuf<int4> brow;
-    DevBuf<unsigned> bar;               // arrivals, exits, error
+    DevBuf<unsigned> bar;               // arrivals, exits
     DevBuf<int> bslot;                  // per colour sweep_rounds x sweep_grid: the batch of a CTA, or -1
     int sweep_rounds = 1;
     int sweep_grid = 0;                 // CTAs of k_schwarz_sweep (0: one launch per colour)
