@@ -587,7 +587,6 @@ __global__ void __launch_bounds__(kSwThreads, 1)
     extern __shared__ __align__(16) unsigned char col_smem[];
     // this CTA's first batch of every colour (np = 0: none); the last entry: a later round's
     __shared__ SchwarzImpl::BatchDesc sbd[kSwMaxColours + 1];
-    __shared__ int s_ok;
     const int tid = threadIdx.x, G = (int)gridDim.x;
     const int sub = tid & (kRowLanes - 1), li = tid / kRowLanes;   // residual role: lane of row li
     constexpr int kPass = kSwThreads / kRowLanes;
@@ -602,8 +601,8 @@ __global__ void __launch_bounds__(kSwThreads, 1)
         else
             sbd[tid].np = 0;
     }
-    if (tid == 0) s_ok = *reinterpret_cast<volatile unsigned*>(P.err) == 0;
-    __syncthreads();
+    // one answer for the CTA, now and at each barrier: its threads leave together
+    bool ok = __syncthreads_and(tid != 0 || *reinterpret_cast<volatile unsigned*>(P.err) == 0);
     int64_t loaded = -1;                                           // the inverse in shared memory
     // state fetched ahead of the barrier: the residual row's entries, its right-hand side, DOF
     int c[kSwPre], k0 = 0, k1 = 0;
@@ -680,7 +679,6 @@ __global__ void __launch_bounds__(kSwThreads, 1)
         return r < P.ncol ? r : 2 * P.ncol - 1 - r;
     };
     const int steps = 2 * P.ncol * P.runs;
-    bool ok = s_ok != 0;
     // step -1 only fetches for step 0 (one code path: registers are what this kernel is short of)
 #pragma unroll 1
     for (int s = -1; ok && s < steps; s++) {
@@ -713,9 +711,10 @@ __global__ void __launch_bounds__(kSwThreads, 1)
             load_inverse(nx);
         }
         if (s < 0) continue;
+        bool in = true;
         if (tid == kSwThreads - 1) {
             const unsigned want = (unsigned)(s + 1) * (unsigned)G;
-            bool in = false;
+            in = false;
 #pragma unroll 1
             for (int i = 0; i < P.spins && !in; i++) {
                 unsigned now;
@@ -723,10 +722,8 @@ __global__ void __launch_bounds__(kSwThreads, 1)
                 in = now >= want;
                 if (!in && i > 64) __nanosleep(64);
             }
-            s_ok = in;
         }
-        __syncthreads();
-        ok = s_ok != 0;
+        ok = __syncthreads_and(in);
     }
     cp_async_wait<0>();
     if (tid == 0) {

@@ -56,3 +56,27 @@ def test_inverses_in_global_memory(ctx, monkeypatch):
     z = S.mg.mvMul(v)
     runs_out(monkeypatch, lambda: S.mg.mvMul(v))
     assert np.array_equal(S.mg.mvMul(v), z)
+
+
+@pytest.mark.parametrize("cells,partitions", [(24, 12), (72, 36)])   # CTAs without a batch in some colours
+def test_waits_that_run_out_at_different_steps(ctx, monkeypatch, cells, partitions):
+    """Few polls: CTAs give up at different steps, each as a whole.  Every call ends,
+    with the usual bits or with the error."""
+    th = TaylorHoodSpace(cells, cells)
+    R, Cc, V, _ = velocity_block(th)
+    A = DeviceMatrix(th.nv, th.nv, R, Cc, V, ctx)
+    rng = np.random.default_rng(64)
+    b, x = rng.standard_normal(th.nv), rng.standard_normal(th.nv)
+    sm = SchwarzSmoother(3, ColoredCartesianSchwarz(A, th.velocity, (partitions, partitions), 1, DirectSolver(), 0.9))
+    good = sm.smooth(A, b, x)
+    ends = {"bits": 0, "error": 0}
+    for spins in (1, 2, 3, 5, 8, 12, 20, 40) * 4:
+        monkeypatch.setenv("JFEM_SCHWARZ_SWEEP_SPINS", str(spins))
+        try:
+            assert np.array_equal(sm.smooth(A, b, x), good)
+            ends["bits"] += 1
+        except N.JfgError as e:
+            assert e.status == N.ERR_CUDA and "ran out" in str(e)
+            ends["error"] += 1
+    monkeypatch.delenv("JFEM_SCHWARZ_SWEEP_SPINS")
+    assert ends["error"] > 0 and np.array_equal(sm.smooth(A, b, x), good)
