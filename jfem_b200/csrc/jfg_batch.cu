@@ -580,10 +580,10 @@ __global__ void __launch_bounds__(NT, NT > 512 ? 1 : 1024 / NT) k_batch_onchip(c
     const int nrow = cnt > tid ? (cnt - 1 - tid) / NT + 1 : 0;     // rows of this thread
     // every row of the warp regular (or absent): the passes run without a branch
     const bool plain = __all_sync(0xffffffffu, regular == (1u << nrow) - 1u);
-    // the halo in front too: a lower neighbour that owns fewer than H rows fills it in
-    // part only, and the absent rows' products read all of it (0 * what a kernel before left)
-    for (int t = tid; t < H; t += NT) zs[t] = 0.f;
-    for (int t = cnt + H + tid; t < NT * RPT + 2 * H; t += NT) zs[t] = 0.f;   // read by absent rows: finite
+    // what no row writes is read all the same, against zero matrix values, by absent
+    // rows: behind the rows, and in front of them the halo, which a lower neighbour
+    // with fewer than H rows fills in part only
+    for (int t = tid; t < NT * RPT + 2 * H; t += NT) zs[t] = 0.f;
     const float* zc = zs + H + tid;
     const float* z3[3] = {zc - str, zc, zc + str};
     cl.sync();                                      // every CTA runs before a halo store reaches it
