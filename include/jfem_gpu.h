@@ -47,7 +47,12 @@ const char* jfg_last_error(jfg_ctx* ctx);
 int jfg_synchronize(jfg_ctx* ctx);
 /* Frees the grow-only scratch the sparse products keep in the context (up to
  * ~70 bytes per product of the largest row chunk, i.e. a few GB after a
- * Galerkin product of a 1 M-row matrix).  Not part of the reference surface. */
+ * Galerkin product of a 1 M-row matrix), and the device blocks the library
+ * keeps between owners: what matrices, hierarchies and other objects give back,
+ * up to 1 GB per device for all contexts of the process, in blocks of up to
+ * 256 MB.  jfg_destroy frees these blocks too, and so does an allocation of the
+ * library that the device refuses at first; allocations of other libraries in
+ * the process do not.  Not part of the reference surface. */
 int jfg_release_scratch(jfg_ctx* ctx);
 /* The context's CUDA stream (cudaStream_t) for callers that time or order work. */
 void* jfg_stream(jfg_ctx* ctx);
