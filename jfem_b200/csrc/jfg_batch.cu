@@ -751,7 +751,6 @@ struct jfg_batch {
         size_t smem = 0;
         cudaStream_t st = nullptr;
         cudaEvent_t done = nullptr;
-        int dev = 0;
     };
     std::vector<int> oc_cluster;
     std::vector<OnchipSys> oc_host;
@@ -764,10 +763,7 @@ struct jfg_batch {
     {
         for (auto& l : oc) {
             if (l.done) cudaEventDestroy(l.done);
-            if (!l.st) continue;
-            cudaStreamSynchronize(l.st);          // a call that failed half-way has not joined it
-            jfg::pool_drop_stream(l.dev, l.st);
-            cudaStreamDestroy(l.st);
+            if (l.st) cudaStreamDestroy(l.st);
         }
         if (oc_fork) cudaEventDestroy(oc_fork);
     }
@@ -1048,8 +1044,6 @@ void plan_onchip(jfg_batch* b)
         JFG_CUDA(cudaEventCreateWithFlags(&b->oc_fork, cudaEventDisableTiming));
         for (auto& l : b->oc) {
             JFG_CUDA(cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking));
-            l.dev = jfg::ctx_device(b->ctx);
-            jfg::pool_add_stream(l.dev, l.st);
             JFG_CUDA(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
         }
     }
@@ -1061,24 +1055,30 @@ void plan_onchip(jfg_batch* b)
 }
 
 // The on-chip systems: one launch per cluster size, each on its own stream
-// between the context stream's work before and after.
+// between the context stream's work before and after.  A failure half-way waits for
+// what it has launched: device blocks are released on the word of the context's stream.
 void enqueue_onchip(jfg_batch* b, int steps, const jfg_batch_opts& o)
 {
     if (b->oc.empty()) return;
     cudaStream_t st = jfg::ctx_stream(b->ctx);
     JFG_CUDA(cudaEventRecord(b->oc_fork, st));
-    for (auto& l : b->oc) {
-        OnchipParams P = {b->oc_sys.p, b->oc_order.p + l.first, steps, o.rtol, o.inner_rtol, o.inner_max, o.max_refine,
-                          b->iters.p, b->relres.p, b->refines.p, b->status.p};
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute at[1];
-        onchip_config(cfg, at, l.var, l.C, l.smem, l.count, l.st);
-        JFG_CUDA(cudaStreamWaitEvent(l.st, b->oc_fork, 0));
-        JFG_CUDA(cudaLaunchKernelEx(&cfg, onchip_kernel(l.var), P));
-        jfg::note_launch();
-        JFG_CUDA(cudaEventRecord(l.done, l.st));
+    try {
+        for (auto& l : b->oc) {
+            OnchipParams P = {b->oc_sys.p, b->oc_order.p + l.first, steps, o.rtol, o.inner_rtol, o.inner_max, o.max_refine,
+                              b->iters.p, b->relres.p, b->refines.p, b->status.p};
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute at[1];
+            onchip_config(cfg, at, l.var, l.C, l.smem, l.count, l.st);
+            JFG_CUDA(cudaStreamWaitEvent(l.st, b->oc_fork, 0));
+            JFG_CUDA(cudaLaunchKernelEx(&cfg, onchip_kernel(l.var), P));
+            jfg::note_launch();
+            JFG_CUDA(cudaEventRecord(l.done, l.st));
+        }
+        for (auto& l : b->oc) JFG_CUDA(cudaStreamWaitEvent(st, l.done, 0));
+    } catch (...) {
+        for (auto& l : b->oc) cudaStreamSynchronize(l.st);
+        throw;
     }
-    for (auto& l : b->oc) JFG_CUDA(cudaStreamWaitEvent(st, l.done, 0));
 }
 
 }  // namespace

@@ -58,8 +58,8 @@ void allow_smem(PerDevice& once, K kern, size_t bytes)
 void* pool_alloc(size_t bytes, int* dev);
 void pool_free(void* p, size_t bytes, int dev) noexcept;
 void pool_trim(int dev) noexcept;
-// Every stream that the library launches on is made known to the pool before its
-// first use and taken off the list before it is destroyed.
+// A context's stream is made known to the pool before its first use and taken off
+// the list before it is destroyed; work on any other stream is joined into it.
 void pool_add_stream(int dev, cudaStream_t st);
 void pool_drop_stream(int dev, cudaStream_t st) noexcept;
 // Around each stream capture: no release waits for a stream meanwhile.

@@ -5,13 +5,13 @@
 // 263 k-row matrix.  A released block is kept, by device and size class, and
 // handed to the next allocation of that class.
 //   * Safety: a block may be handed out once no queued work uses it any more.  All
-//     work of the library runs on the streams it has made (one per context, and
-//     those of the batched launches), so a release waits for these.  It does not
-//     wait for the device: that is an error, and breaks the capture, while any
-//     stream of the device is being captured, whoever's it is.  While a solver of
-//     this process captures (CaptureScope), or one of these streams is found
-//     capturing, the release is a plain cudaFree, which other threads may call
-//     during a thread-local capture.
+//     work of the library runs on its contexts' streams (what a batched call runs
+//     beside it is joined before the call returns), so a release waits for these,
+//     1.5 us a context when they are idle.  It does not wait for the device: that
+//     is an error, and breaks the capture, while any stream of the device is being
+//     captured, whoever's it is.  While a solver of this process captures
+//     (CaptureScope), or one of these streams is found capturing, the release is a
+//     plain cudaFree, which other threads may call during a thread-local capture.
 //   * Bound: at most kPoolCap bytes per device are kept, in blocks of at most
 //     kPoolBlock; what does not fit is freed at once.  pool_trim gives everything
 //     back (jfg_release_scratch, jfg_destroy, and before an allocation that the
