@@ -13,10 +13,12 @@
 //     (CaptureScope), or one of these streams is found capturing, the release is a
 //     plain cudaFree, which other threads may call during a thread-local capture.
 //   * Bound: at most kPoolCap bytes per device are kept, in blocks of at most
-//     kPoolBlock; what does not fit is freed at once.  pool_trim gives everything
-//     back (jfg_release_scratch, jfg_destroy, and before an allocation that the
-//     device refuses is tried again).
+//     kPoolBlock (larger ones are freed at once); beyond that the block kept for
+//     longest goes, or a pool filled by other sizes would keep nothing any more.
+//     pool_trim gives everything back (jfg_release_scratch, jfg_destroy, and before
+//     an allocation that the device refuses is tried again).
 #include <algorithm>
+#include <list>
 #include <map>
 #include <mutex>
 
@@ -28,10 +30,47 @@ namespace {
 constexpr size_t kPoolCap = (size_t)1 << 30;
 constexpr size_t kPoolBlock = (size_t)256 << 20;
 
+struct Block {
+    size_t c;                                      // class
+    void* p;
+};
+struct Kept {                                      // the free blocks of a device
+    std::list<Block> all;                          // oldest first
+    std::map<size_t, std::vector<std::list<Block>::iterator>> of;   // by class, oldest first
+    size_t bytes = 0;
+
+    void* take(size_t c)                           // the newest of a class
+    {
+        auto f = of.find(c);
+        if (f == of.end() || f->second.empty()) return nullptr;
+        auto b = f->second.back();
+        f->second.pop_back();
+        void* p = b->p;
+        all.erase(b);
+        bytes -= c;
+        return p;
+    }
+    void put(size_t c, void* p)
+    {
+        auto& v = of[c];
+        v.reserve(v.size() + 1);                   // nothing throws after the block is in the list
+        all.push_back(Block{c, p});
+        v.push_back(std::prev(all.end()));
+        bytes += c;
+    }
+    void* drop_oldest()
+    {
+        const Block b = all.front();
+        auto& v = of[b.c];
+        v.erase(v.begin());
+        all.pop_front();
+        bytes -= b.c;
+        return b.p;
+    }
+};
 struct Pool {
     std::mutex m;
-    std::map<std::pair<int, size_t>, std::vector<void*>> blocks;   // (device, class) -> free blocks
-    std::map<int, size_t> kept;                                    // bytes per device
+    std::map<int, Kept> of;
 };
 Pool& pool()
 {
@@ -97,13 +136,7 @@ void* pool_alloc(size_t bytes, int* dev)
     Pool& p = pool();
     if (c <= kPoolBlock) {
         std::lock_guard<std::mutex> g(p.m);
-        auto it = p.blocks.find({*dev, c});
-        if (it != p.blocks.end() && !it->second.empty()) {
-            void* b = it->second.back();
-            it->second.pop_back();
-            p.kept[*dev] -= c;
-            return b;
-        }
+        if (void* b = p.of[*dev].take(c)) return b;
     }
     const size_t size = c <= kPoolBlock ? c : bytes;      // a block that is never kept is not rounded up
     void* b = nullptr;
@@ -128,12 +161,16 @@ void pool_free(void* b, size_t bytes, int dev) noexcept
     if (c <= kPoolBlock) {
         try {
             if (wait_streams(dev)) {
-                std::lock_guard<std::mutex> g(p.m);
-                if (p.kept[dev] + c <= kPoolCap) {
-                    p.blocks[{dev, c}].push_back(b);
-                    p.kept[dev] += c;
-                    return;
+                std::vector<void*> old;
+                {
+                    std::lock_guard<std::mutex> g(p.m);
+                    Kept& k = p.of[dev];
+                    old.reserve(k.all.size());
+                    k.put(c, b);
+                    while (k.bytes > kPoolCap) old.push_back(k.drop_oldest());
                 }
+                for (void* o : old) cudaFree(o);
+                return;
             }
         } catch (...) {
         }
@@ -175,12 +212,8 @@ void pool_trim(int dev) noexcept
     DeviceGuard on(dev);
     Pool& p = pool();
     std::lock_guard<std::mutex> g(p.m);
-    for (auto& kv : p.blocks)
-        if (kv.first.first == dev) {
-            for (void* b : kv.second) cudaFree(b);
-            kv.second.clear();
-        }
-    p.kept[dev] = 0;
+    Kept& k = p.of[dev];
+    while (!k.all.empty()) cudaFree(k.drop_oldest());
 }
 
 }  // namespace jfg
